@@ -175,6 +175,9 @@ struct EpiResidual {
 template <int SIGN, int BLOCK, int MINB, class Lk, class Epi>
 __global__ void __launch_bounds__(BLOCK, MINB) k_hop(Geom g, Lk U, int par, SpinorF64 in, Epi epi, RedBuf red) {
     extern __shared__ double2 stage[];  // Epi::NPRE x 12 x BLOCK
+    chain_begin();
+    U.p = chained(U.p);
+    in.p = chained(in.p);
     if (epi.skip()) return;
     const int i = blockIdx.x * BLOCK + threadIdx.x;
     double v[Epi::NRED > 0 ? Epi::NRED : 1];
@@ -229,9 +232,11 @@ void launch_variant(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin
                     cudaStream_t s) {
     dim3 grid((g.Vh + BLOCK - 1) / BLOCK);
     if (sign > 0)
-        k_hop<1, BLOCK, MINB><<<grid, BLOCK, hop_smem<1, BLOCK, MINB, Lk, Epi>(), s>>>(g, L, par, sin, epi, rb);
+        launch_chain(g.chain, k_hop<1, BLOCK, MINB, Lk, Epi>, grid, BLOCK, hop_smem<1, BLOCK, MINB, Lk, Epi>(), s, g, L,
+                     par, sin, epi, rb);
     else
-        k_hop<-1, BLOCK, MINB><<<grid, BLOCK, hop_smem<-1, BLOCK, MINB, Lk, Epi>(), s>>>(g, L, par, sin, epi, rb);
+        launch_chain(g.chain, k_hop<-1, BLOCK, MINB, Lk, Epi>, grid, BLOCK, hop_smem<-1, BLOCK, MINB, Lk, Epi>(), s, g, L,
+                     par, sin, epi, rb);
 }
 
 // Launch shapes the autotuner chooses from (HopVariant in kernels.h):

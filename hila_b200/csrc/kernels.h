@@ -9,6 +9,45 @@
 
 namespace hw {
 
+// Launch of a kernel of a chain on one stream.  With `chain` it may become resident while the
+// kernel before it drains (programmatic dependent launch); it begins with chain_begin(), which
+// waits for that kernel to complete before anything is read or written.  Between the two hops
+// of an operator call this hides the launch and the drain: one even-odd apply took 12.4 -> 8.5
+// us at 8^4, 18.6 -> 15.5 us at 16^4 and 103 -> 98 us at 24^4 (18 reals).  Not in the body of a
+// CUDA-graph loop, where the early residents of the next kernel crowd the SMs that drain
+// first: an FP64 CG iteration took 52 -> 63 us at 16^4 and was no faster at 32^4.
+template <class... KArgs, class... Args>
+inline void launch_chain(bool chain, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                         const Args &...args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = chain ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+#ifdef __CUDACC__
+// First statement of every kernel launched by launch_chain: waits for the kernels before it
+// on the stream, then lets the next one become resident (its own wait holds it back).
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// A pointer that loads through the read-only path (which the compiler may move over the
+// wait) start from: its value is known only after chain_begin().
+template <class T>
+__device__ __forceinline__ T *chained(T *p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+#endif
+
 constexpr int kHopBlock = 128;
 constexpr int kHopMinBlock = 128;  // smallest block of any hop launch shape (sizes reduction buffers)
 constexpr int kHopVariants = 3;

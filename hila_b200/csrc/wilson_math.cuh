@@ -338,6 +338,7 @@ struct Geom {
     int sy, sz, st; // checkerboard strides of y, z, t: lxh, lxh*Ly, lxh*Ly*Lz
     int tap;        // 1: fermion values crossing the t boundary are negated
     int hop_variant;  // launch shape of the FP64 hop kernels (host-side choice, see dslash_f64.cu)
+    int chain;        // 1: the FP64 hop may overlap the drain of the kernel before it (launch_chain)
     FastDiv dx, dy, dz;  // division by lxh, Ly, Lz
 };
 
@@ -351,6 +352,7 @@ inline void geom_setup(Geom &g, const int dims[4], int tap) {
     g.st = g.lxh * dims[1] * dims[2];
     g.tap = tap ? 1 : 0;
     g.hop_variant = 0;
+    g.chain = 1;
     g.dx.init((unsigned)g.lxh);
     g.dy.init((unsigned)dims[1]);
     g.dz.init((unsigned)dims[2]);

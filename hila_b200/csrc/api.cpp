@@ -65,6 +65,10 @@ int tune_hop(hw_lattice *lat, const hw_gauge *G) {
         lat->g.hop_variant = (v >= 0 && v < kHopVariants) ? v : 0;
         return HW_OK;
     }
+    if (lat->Vh <= kHopSplitSites) {
+        lat->g.hop_variant = 3;
+        return HW_OK;
+    }
     int rc;
     if ((rc = ensure_workspace(lat)) != HW_OK) return rc;
     hw_context *ctx = lat->ctx;
@@ -79,7 +83,7 @@ int tune_hop(hw_lattice *lat, const hw_gauge *G) {
     };
     float best = 1e30f;
     int best_v = 0;
-    for (int v = 0; v < kHopVariants; v++) {
+    for (int v = 0; v < kHopVariants - 1; v++) {
         Geom g = lat->g;
         g.hop_variant = v;
         for (int k = 0; k < 2; k++) apply(g);

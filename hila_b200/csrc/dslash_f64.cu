@@ -25,7 +25,8 @@ __host__ __device__ __forceinline__ SpinorF64 sp(HalfF64 h) { return SpinorF64{h
 // shared memory with cp.async when the thread starts, so their HBM reads overlap
 // the hop instead of following it.  An epilogue with NPRE > 0 names them in
 // pre(k) and reads them from stg (component c of operand k at stg.p[(k*12 + c)
-// * BLOCK + threadIdx.x]; `stg.stride` = BLOCK, index ix = threadIdx.x).
+// * BLOCK + threadIdx.x]; `stg.stride` = BLOCK, index ix = threadIdx.x).  spin3 is the same
+// epilogue on one spin of a site, with its NOWN own-site operands (own(k)) loaded.
 // (cp_async16 and cp_async_wait_all: storage.cuh)
 // operand k of a staged epilogue as a field over the block's threads
 __device__ __forceinline__ SpinorF64 staged(double2 *stage, int block, int k) {
@@ -44,6 +45,15 @@ struct EpiScale {
 #pragma unroll
         for (int c = 0; c < 12; c++) acc.s[c / 3][c % 3] = a * acc.s[c / 3][c % 3];
         out.store(i, acc);
+    }
+    static constexpr int NOWN = 0;
+    __device__ SpinorF64 own(int) const { return out; }
+    __device__ void spin3(int i, int s, const Cx<double> (&acc)[3], const Cx<double> (&)[1][3], double *) const {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const Cx<double> v = a * acc[k];
+            out.p[(size_t)(3 * s + k) * out.stride + i] = make_double2(v.re, v.im);
+        }
     }
 };
 
@@ -87,11 +97,25 @@ struct EpiXpay {
             for (int c = 0; c < 12; c++) zero[(size_t)c * out.stride + i] = make_double2(0.0, 0.0);
         if (RED) red[0] = n2;
     }
+    static constexpr int NOWN = 1;
+    __device__ SpinorF64 own(int) const { return x; }
+    __device__ void spin3(int i, int s, const Cx<double> (&acc)[3], const Cx<double> (&o)[1][3], double *red) const {
+        double n2 = 0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const Cx<double> v = dscale(d, o[0][k]) + b * acc[k];
+            store_c(out, 3 * s + k, i, v);
+            if (zero) zero[(size_t)(3 * s + k) * out.stride + i] = make_double2(0.0, 0.0);
+            n2 += norm2(v);
+        }
+        if (RED) red[0] = n2;
+    }
     __device__ void operator()(const double *tot) {
         st->pAp = tot[0];
         if (!(tot[0] > 0.0) || !isfinite(tot[0])) {
             st->status = CG_BREAKDOWN;
             st->alpha = 0.0;
+            st->do_pupdate = 0;
         } else {
             st->alpha = st->rr / tot[0];
         }
@@ -120,6 +144,21 @@ struct EpiCgUpdate {
             Cx<double> rv = load_c(rs, c, ix) - alpha * ddp;
             store_c(r, c, i, rv);
             store_c(x, c, i, load_c(x, c, i) + alpha * load_c(p, c, i));
+            n2 += norm2(rv);
+        }
+        red[0] = n2;
+    }
+    static constexpr int NOWN = 4;
+    __device__ SpinorF64 own(int k) const { return k == 0 ? Dp : k == 1 ? r : k == 2 ? x : p; }
+    __device__ void spin3(int i, int s, const Cx<double> (&acc)[3], const Cx<double> (&o)[4][3], double *red) const {
+        const double alpha = st->alpha;
+        double n2 = 0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const Cx<double> ddp = dscale(d, o[0][k]) + b * acc[k];
+            const Cx<double> rv = o[1][k] - alpha * ddp;
+            store_c(r, 3 * s + k, i, rv);
+            store_c(x, 3 * s + k, i, o[2][k] + alpha * o[3][k]);
             n2 += norm2(rv);
         }
         red[0] = n2;
@@ -166,6 +205,20 @@ struct EpiResidual {
         red[0] = n2;
         red[1] = d2;
     }
+    static constexpr int NOWN = 2;
+    __device__ SpinorF64 own(int k) const { return k == 0 ? x : src; }
+    __device__ void spin3(int i, int s, const Cx<double> (&acc)[3], const Cx<double> (&o)[2][3], double *red) const {
+        double n2 = 0, d2 = 0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const Cx<double> v = o[1][k] - (dscale(d, o[0][k]) + b * acc[k]);
+            if (res.p) store_c(res, 3 * s + k, i, v);
+            n2 += norm2(v);
+            d2 += norm2(o[1][k]);
+        }
+        red[0] = n2;
+        red[1] = d2;
+    }
     __device__ void operator()(const double *tot) {
         st->res_num2 = tot[0];
         st->res_den2 = tot[1];
@@ -205,6 +258,142 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_hop(Geom g, Lk U, int par, Spin
     if constexpr (Epi::NRED > 0) grid_reduce<Epi::NRED, BLOCK>(v, red.partials, red.ticket, epi);
 }
 
+// One term of the hop at one site: the half spinors v0, v1 of U_mu(x) P in(x + mu)
+// (BACK: of U_mu(x - mu)^dag P in(x - mu)), computed as hop_dir_lean does.
+template <int MU, int SIGN, bool BACK, class Lk>
+__device__ __forceinline__ void hop_term(const Geom &g, const Lk &U, int par, int i, const SpinorF64 &in,
+                                         Cx<double> v0[3], Cx<double> v1[3]) {
+    constexpr int S = BACK ? -SIGN : SIGN;
+    const SiteNbrs n = site_neighbours(g, i, par);
+    const int j = BACK ? n.bwd[MU] : n.fwd[MU];
+    Cx<double> h0[3], h1[3];
+    Spinor<double> w;
+    in.load(j, w);
+    Su3<double> u;
+    if (BACK)
+        U.load(1 - par, MU, j, u);
+    else
+        U.load(par, MU, i, u);
+    project<MU, S>(w, h0, h1);
+    if (MU == 3) {
+        const double sg = (BACK ? n.tbwd_wrap : n.tfwd_wrap) ? -1.0 : 1.0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            h0[k] = sg * h0[k];
+            h1[k] = sg * h1[k];
+        }
+    }
+    if (BACK) {
+        su3_adj_mul(u, h0, v0);
+        su3_adj_mul(u, h1, v1);
+    } else {
+        su3_mul(u, h0, v0);
+        su3_mul(u, h1, v1);
+    }
+}
+
+// acc + phase * v, phase code 0: 1, 1: i, 2: -1, 3: -i
+template <int PH>
+__device__ __forceinline__ Cx<double> add_phase(Cx<double> acc, Cx<double> v) {
+    if constexpr (PH == 0) return acc + v;
+    if constexpr (PH == 1) return acc + mul_i(v);
+    if constexpr (PH == 2) return acc - v;
+    return acc - mul_i(v);
+}
+
+constexpr int kSplitSites = 32;                 // sites of a block: one per lane
+constexpr int kSplitBlock = 8 * kSplitSites;    // a warp per term of the hop
+using SplitTerms = double2[8][6][kSplitSites];  // [term][3 * half spinor + colour][site]
+
+// spin S of E_{mu,+-}(v0, v1) summed over the terms in hop_site's order (the same bits)
+template <int S, int SIGN, int T = 0>
+__device__ __forceinline__ void sum_terms(const SplitTerms &part, int lane, Cx<double> (&acc)[3]) {
+    if constexpr (T < 8) {
+        using P = ProjTable<T / 2, (T & 1) ? -SIGN : SIGN>;
+        constexpr int q = S < 2 ? S : (S == 2 ? P::q0 : P::q1);
+        constexpr int ph = S < 2 ? 0 : (S == 2 ? P::ps0 : P::ps1);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const double2 v = part[T][3 * q + k][lane];
+            acc[k] = add_phase<ph>(acc[k], {v.x, v.y});
+        }
+        sum_terms<S, SIGN, T + 1>(part, lane, acc);
+    }
+}
+
+// The hop of a small lattice, eight warps per 32 sites: warp k computes term k (direction k / 2,
+// forward or backward) of the block's sites, the half spinors meet in shared memory, and warp
+// s < 4 sums spin s, in the order of hop_site, and runs the epilogue on it.  A site's loads
+// are all in flight together, where k_hop's thread goes through eight dependent rounds of
+// them, and a lattice of some thousand sites reaches eight times as many SMs.
+template <int SIGN, class Lk, class Epi>
+__global__ void __launch_bounds__(kSplitBlock, 2) k_hop_split(Geom g, Lk U, int par, SpinorF64 in, Epi epi,
+                                                             RedBuf red) {
+    __shared__ SplitTerms part;
+    chain_begin();
+    U.p = chained(U.p);
+    in.p = chained(in.p);
+    if (epi.skip()) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NR = Epi::NRED > 0 ? Epi::NRED : 1;
+    double v[NR];
+#pragma unroll
+    for (int k = 0; k < NR; k++) v[k] = 0.0;
+    const int i = blockIdx.x * kSplitSites + lane;
+    if (i < g.Vh) {
+        Cx<double> v0[3], v1[3];
+        switch (warp) {
+        case 0: hop_term<0, SIGN, false>(g, U, par, i, in, v0, v1); break;
+        case 1: hop_term<0, SIGN, true>(g, U, par, i, in, v0, v1); break;
+        case 2: hop_term<1, SIGN, false>(g, U, par, i, in, v0, v1); break;
+        case 3: hop_term<1, SIGN, true>(g, U, par, i, in, v0, v1); break;
+        case 4: hop_term<2, SIGN, false>(g, U, par, i, in, v0, v1); break;
+        case 5: hop_term<2, SIGN, true>(g, U, par, i, in, v0, v1); break;
+        case 6: hop_term<3, SIGN, false>(g, U, par, i, in, v0, v1); break;
+        default: hop_term<3, SIGN, true>(g, U, par, i, in, v0, v1); break;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            part[warp][k][lane] = make_double2(v0[k].re, v0[k].im);
+            part[warp][3 + k][lane] = make_double2(v1[k].re, v1[k].im);
+        }
+    }
+    // the epilogue's own-site operands travel while the block meets
+    constexpr int NO = Epi::NOWN > 0 ? Epi::NOWN : 1;
+    Cx<double> own[NO][3];
+    const bool mine = warp < 4 && i < g.Vh;
+    if (Epi::NOWN > 0 && mine) {
+#pragma unroll
+        for (int q = 0; q < Epi::NOWN; q++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) own[q][k] = load_c(epi.own(q), 3 * warp + k, i);
+    }
+    __syncthreads();
+    if (mine) {
+        Cx<double> acc[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        if (warp == 0)
+            sum_terms<0, SIGN>(part, lane, acc);
+        else if (warp == 1)
+            sum_terms<1, SIGN>(part, lane, acc);
+        else if (warp == 2)
+            sum_terms<2, SIGN>(part, lane, acc);
+        else
+            sum_terms<3, SIGN>(part, lane, acc);
+        epi.spin3(i, warp, acc, own, v);
+    }
+    if constexpr (Epi::NRED > 0) grid_reduce<Epi::NRED, kSplitBlock>(v, red.partials, red.ticket, epi);
+}
+
+template <class Lk, class Epi>
+void launch_split(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin, const Epi &epi, RedBuf rb,
+                  cudaStream_t s) {
+    dim3 grid((g.Vh + kSplitSites - 1) / kSplitSites);
+    if (sign > 0)
+        launch_chain(g.chain, k_hop_split<1, Lk, Epi>, grid, kSplitBlock, 0, s, g, L, par, sin, epi, rb);
+    else
+        launch_chain(g.chain, k_hop_split<-1, Lk, Epi>, grid, kSplitBlock, 0, s, g, L, par, sin, epi, rb);
+}
+
 // shared memory of the staged epilogue operands.  Near the 48 KB default the kernel is
 // opted in to more, once per instantiation and device (the attribute belongs to the
 // device that is current when it is set; contexts on several GPUs share one process).
@@ -242,12 +431,16 @@ void launch_variant(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin
 // Launch shapes the autotuner chooses from (HopVariant in kernels.h):
 //   0: 128 threads, registers unconstrained   1: 128 threads, <= 128 registers (4 blocks/SM)
 //   2: 256 threads, <= 128 registers
+// and, not timed, 3: k_hop_split, for lattices up to kHopSplitSites
 // (128 threads at <= 102 registers spills about 600 bytes per thread and measured 0.63 of
 // HBM peak against 0.80-0.83 for these.)
 template <class Lk, class Epi>
 void launch_shape(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin, const Epi &epi, RedBuf rb,
                   cudaStream_t s) {
     switch (g.hop_variant) {
+    case 3:
+        launch_split(g, L, par, sign, sin, epi, rb, s);
+        break;
     case 1:
         launch_variant<128, 4>(g, L, par, sign, sin, epi, rb, s);
         break;
@@ -317,7 +510,10 @@ __global__ void __launch_bounds__(kVecBlock) k_cg_init(int Vh, SpinorF64 src, Sp
     grid_reduce<2, kVecBlock>(v, red.partials, red.ticket, fin);
 }
 
-__global__ void __launch_bounds__(kVecBlock) k_cg_pupdate(int Vh, SpinorF64 r, SpinorF64 p, const CgState *st) {
+// Last kernel of every CG loop-body iteration
+__global__ void __launch_bounds__(kVecBlock) k_cg_pupdate(int Vh, SpinorF64 r, SpinorF64 p, const CgState *st,
+                                                          cudaGraphConditionalHandle cond, int use_cond) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) loop_next(st, cond, use_cond);
     if (!st->do_pupdate) return;
     const int i = blockIdx.x * kVecBlock + threadIdx.x;
     if (i >= Vh) return;
@@ -330,15 +526,8 @@ __global__ void __launch_bounds__(kVecBlock) k_cg_pupdate(int Vh, SpinorF64 r, S
     }
 }
 
-// Last node of every CG loop-body iteration: keeps the graph's while loop
-// going only while the solve is running.  It always runs, so the loop ends
-// even when every other body kernel returned early; the iteration counter is
-// bounded by maxiter, so the loop is bounded.
-__global__ void k_loop_control(CgState *st, cudaGraphConditionalHandle cond, int use_cond) {
-    st->do_pupdate = 0;
-    if (st->status == CG_RUNNING && st->iter >= st->maxiter) st->status = CG_MAXITER;
-    if (use_cond) cudaGraphSetConditional(cond, st->status == CG_RUNNING ? 1u : 0u);
-}
+// in a host loop the bodies after the last step must not form p again
+__global__ void k_pupdate_done(CgState *st) { st->do_pupdate = 0; }
 
 __global__ void __launch_bounds__(kVecBlock) k_scale(int Vh, SpinorF64 x, SpinorF64 y, double a) {
     const int i = blockIdx.x * kVecBlock + threadIdx.x;
@@ -462,12 +651,10 @@ void launch_cg_init(int Vh, HalfF64 src, HalfF64 Ax, HalfF64 r, HalfF64 p, doubl
                                                                       sp(p), fin, red);
 }
 
-void launch_cg_pupdate(int Vh, HalfF64 r, HalfF64 p, const CgState *st, cudaStream_t s) {
-    k_cg_pupdate<<<(Vh + kVecBlock - 1) / kVecBlock, kVecBlock, 0, s>>>(Vh, sp(r), sp(p), st);
-}
-
-void launch_loop_control(CgState *st, cudaGraphConditionalHandle cond, int use_cond, cudaStream_t s) {
-    k_loop_control<<<1, 1, 0, s>>>(st, cond, use_cond);
+void launch_cg_pupdate(int Vh, HalfF64 r, HalfF64 p, CgState *st, cudaGraphConditionalHandle cond, int use_cond,
+                       cudaStream_t s) {
+    k_cg_pupdate<<<(Vh + kVecBlock - 1) / kVecBlock, kVecBlock, 0, s>>>(Vh, sp(r), sp(p), st, cond, use_cond);
+    if (!use_cond) k_pupdate_done<<<1, 1, 0, s>>>(st);
 }
 
 void launch_scale(int Vh, HalfF64 x, HalfF64 y, double a, cudaStream_t s) {

@@ -98,11 +98,11 @@ struct CgWorkspace {
     // cached graphs of the last solve
     cudaGraphExec_t init_exec = nullptr, loop_exec = nullptr;
     struct Key {
-        const void *gauge = nullptr, *in = nullptr, *out = nullptr;
+        const void *links = nullptr, *in = nullptr, *out = nullptr, *red = nullptr;  // pointers in the graphs
         double kappa = 0, acc2 = 0, diag = 1;
-        int maxiter = 0, mode = 0;
+        int maxiter = 0, mode = 0, planes = 0;
         bool operator==(const Key &o) const {
-            return gauge == o.gauge && in == o.in && out == o.out && kappa == o.kappa && acc2 == o.acc2 &&
+            return links == o.links && planes == o.planes && red == o.red && in == o.in && out == o.out && kappa == o.kappa && acc2 == o.acc2 &&
                    diag == o.diag && maxiter == o.maxiter && mode == o.mode;
         }
     } key;

@@ -50,7 +50,11 @@ __device__ __forceinline__ T *chained(T *p) {
 
 constexpr int kHopBlock = 128;
 constexpr int kHopMinBlock = 128;  // smallest block of any hop launch shape (sizes reduction buffers)
-constexpr int kHopVariants = 3;
+constexpr int kHopVariants = 4;  // 0..2 timed per lattice, 3 for small lattices (dslash_f64.cu)
+// Sites per parity up to which the hop runs eight warps per 32 sites (k_hop_split): an FP64 CG
+// iteration took 40 -> 30 us at 8^4, 43 -> 39 us at 6x10x14x22 (9240), 43 -> 44 us at 12^4
+// (10368), 52 -> 65 us at 16^4.
+constexpr int kHopSplitSites = 9500;
 
 // Device-resident scalars of one FP64 conjugate-gradient solve
 // (conjugate_gradient.h:55-57 keeps the same quantities on the host).
@@ -64,9 +68,18 @@ struct CgState {
     double res_den2;   //                                |b|^2
     int iter, maxiter;
     int status;        // CG_RUNNING / CG_CONVERGED / CG_MAXITER / CG_BREAKDOWN
-    int do_pupdate;    // set by the CG update, consumed by the p update of the same iteration
+    int do_pupdate;    // whether the iteration's last kernel forms p (its CG update ran)
 };
 enum : int { CG_RUNNING = 0, CG_CONVERGED = 1, CG_MAXITER = 2, CG_BREAKDOWN = 3 };
+
+#ifdef __CUDACC__
+// Keeps a graph's while loop going while the solve runs: called by one thread of an iteration's
+// last kernel (the kernel always runs, so the loop ends even when the others returned early;
+// the iteration counter is bounded by maxiter, so the loop is bounded).
+__device__ __forceinline__ void loop_next(const CgState *st, cudaGraphConditionalHandle cond, int use_cond) {
+    if (use_cond) cudaGraphSetConditional(cond, st->status == CG_RUNNING ? 1u : 0u);
+}
+#endif
 
 // Work buffers for one grid reduction: partial sums and the arrival ticket.
 struct RedBuf {
@@ -113,11 +126,10 @@ void launch_hop_residual(const Geom &g, const GaugeF64 &U, int par, int sign, Ha
 // CG start: r = src - Ax (Ax may be null: x = 0), p = r; sets rr, src_norm2, target_rr, status
 void launch_cg_init(int Vh, HalfF64 src, HalfF64 Ax, HalfF64 r, HalfF64 p, double acc2, int maxiter,
                     CgState *st, const RedBuf &red, cudaStream_t s);
-// p = r + beta p  (beta from st)
-void launch_cg_pupdate(int Vh, HalfF64 r, HalfF64 p, const CgState *st, cudaStream_t s);
-// end of a loop-body iteration: clears do_pupdate, enforces maxiter and (use_cond)
-// keeps the graph while loop going while st->status == CG_RUNNING
-void launch_loop_control(CgState *st, cudaGraphConditionalHandle cond, int use_cond, cudaStream_t s);
+// end of a loop-body iteration: p = r + beta p (beta from st) and, with use_cond, the graph's
+// while loop goes on while st->status == CG_RUNNING
+void launch_cg_pupdate(int Vh, HalfF64 r, HalfF64 p, CgState *st, cudaGraphConditionalHandle cond, int use_cond,
+                       cudaStream_t s);
 // y = a * x
 void launch_scale(int Vh, HalfF64 x, HalfF64 y, double a, cudaStream_t s);
 

@@ -9,8 +9,8 @@
 //   K3  t    = H^{oe}_- Dp
 //   K4  DDp  = Dp - kappa^2 H^{eo}_- t; x += alpha p; r -= alpha DDp
 //                                             + |r|^2 -> beta, convergence
-//   P   p    = r + beta p
-// followed by a one-thread control kernel.  alpha, beta and the stopping
+//   P   p    = r + beta p, and the loop's condition
+// alpha, beta and the stopping
 // decision stay in device memory.  The body is captured into the body graph
 // of a CUDA-graph WHILE node, so a whole solve is one graph launch and one
 // host synchronisation; the explicit FP64 residual check is appended to the
@@ -60,13 +60,14 @@ struct F64Solve {
     }
 
     void enqueue_body(cudaGraphConditionalHandle cond, int use_cond) {
-        launch_hop_scale(lat->g, G->U(), 1, +1, w->p.h(), w->t.h(), 1.0, st, s);
-        launch_hop_xpay(lat->g, G->U(), 0, +1, w->t.h(), w->p.h(), w->Dp.h(), -kappa * kappa, st, &red, s, diag);
-        launch_hop_scale(lat->g, G->U(), 1, -1, w->Dp.h(), w->t.h(), 1.0, st, s);
-        launch_hop_cg_update(lat->g, G->U(), 0, -1, w->t.h(), w->Dp.h(), w->r.h(), x, w->p.h(), -kappa * kappa, st,
+        Geom g = lat->g;
+        g.chain = 0;  // in the body of a graph loop (kernels.h)
+        launch_hop_scale(g, G->U(), 1, +1, w->p.h(), w->t.h(), 1.0, st, s);
+        launch_hop_xpay(g, G->U(), 0, +1, w->t.h(), w->p.h(), w->Dp.h(), -kappa * kappa, st, &red, s, diag);
+        launch_hop_scale(g, G->U(), 1, -1, w->Dp.h(), w->t.h(), 1.0, st, s);
+        launch_hop_cg_update(g, G->U(), 0, -1, w->t.h(), w->Dp.h(), w->r.h(), x, w->p.h(), -kappa * kappa, st,
                              red, s, diag);
-        launch_cg_pupdate(lat->g.Vh, w->r.h(), w->p.h(), st, s);
-        launch_loop_control(st, cond, use_cond, s);
+        launch_cg_pupdate(g.Vh, w->r.h(), w->p.h(), st, cond, use_cond, s);
     }
 
     // explicit FP64 residual of the system being solved -> st->res_num2 / res_den2
@@ -140,7 +141,9 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
     S.red = ctx->red();
 
     CgWorkspace::Key key;
-    key.gauge = S.G;
+    key.links = S.G->U().p;
+    key.planes = S.G->U().planes;
+    key.red = S.red.partials;
     key.in = S.mode == MODE_SOLVE ? (const void *)S.b.p : (const void *)S.in.p;
     key.out = S.x.p;
     key.kappa = S.kappa;
@@ -208,7 +211,7 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
             S.enqueue_check();
         }
         if ((rc = read_state(ctx)) != HW_OK) return rc;
-        true_res = h->res_den2 > 0 ? std::sqrt(h->res_num2 / h->res_den2) : 0.0;
+            true_res = h->res_den2 > 0 ? std::sqrt(h->res_num2 / h->res_den2) : 0.0;
     }
     HW_CUDA(cudaEventRecord(ctx->ev1, S.s));
     HW_CUDA(cudaEventSynchronize(ctx->ev1));
@@ -223,11 +226,11 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
         R->rr_relative = h->src_norm2 > 0 ? h->rr / h->src_norm2 : 0.0;
         R->true_residual = true_res;
         R->seconds = ms * 1e-3;
-        // kernels per phase: init = [2 for M^dag b] + 4 (A x0) + 1; body = 6; check = 2 (M x) or 4
+        // kernels per phase: init = [2 for M^dag b] + 4 (A x0) + 1; body = 5; check = 2 (M x) or 4
         const long init_k = (S.mode == MODE_SOLVE ? 2 : 0) + 5;
         const long check_k = S.mode == MODE_SOLVE ? 2 : 4;
         const long bodies = use_graph ? (long)h->iter + restarts + 1 : host_bodies;
-        R->kernel_launches = (int)(init_k + 6 * bodies + check_k * (1 + restarts));
+        R->kernel_launches = (int)(init_k + 5 * bodies + check_k * (1 + restarts));
         if (h->status == CG_BREAKDOWN)
             R->status = HW_ERR_BREAKDOWN;
         else if (h->status == CG_MAXITER || (P.true_residual && true_res > P.accuracy))

@@ -1,0 +1,83 @@
+"""The FP64 hop of small lattices (eight warps per 32 sites) against the one-thread-per-site
+kernel, and the loop graphs of the unpreconditioned and staggered CG on consecutive sources, at
+the edges of their groups of 32 sites and blocks of 128.
+
+Two solves that stop at |b - A x| / |b| <= acc differ by at most 2 acc |A^-1| |A| |x|; the
+condition numbers here are below 20 for M (kappa 0.12) and 400 for its normal system, so
+1e-8 bounds the solutions at acc = 1e-11.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ACC = 1e-11
+SOL_TOL = 1e-8
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+# sites per parity: 8 (a quarter of a group), 24, 96, 240, 2048, 9240 (near the limit of the rule)
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 2, 2, 6), (4, 2, 6, 4), (6, 4, 2, 10), (8, 8, 8, 8),
+                                  (6, 10, 14, 22)])
+@pytest.mark.parametrize("link_format", [18, 12])
+def test_split_hop(hw, ctx, oracle, monkeypatch, dims, link_format):
+    """Every epilogue of the small lattices' hop: the same bits as the one-thread-per-site kernel
+    for operators, and the same solutions (the sums of |.|^2 are formed in another order)."""
+    U = oracle.gen_links(dims, 0.3, 5)
+    src, guess = oracle.gen_spinor(dims, 6, oracle.ALL), 0.1 * oracle.gen_spinor(dims, 7, oracle.EVEN)
+
+    def run(variant):
+        if variant is None:
+            monkeypatch.delenv("HW_HOP_VARIANT", raising=False)
+        else:
+            monkeypatch.setenv("HW_HOP_VARIANT", variant)
+        lat = hw.Lattice(ctx, dims)  # the launch shape is chosen per lattice
+        G = hw.GaugeField(lat, U, link_format)
+        D, F = hw.Dirac_Wilson_evenodd(0.12, G), hw.Dirac_Wilson(0.12, G)
+        b, bits, sols = hw.Field(lat, src), [], []
+        for op in (D.apply, D.dagger, F.apply, F.dagger, hw.Hasenbusch_operator(D, 0.3).dagger):
+            o = hw.Field(lat, guess, oracle.ALL)
+            op(b, o)
+            bits.append(o.download())
+        for parity in (hw.EVEN, hw.ODD):
+            for sign in (1, -1):
+                for set_ in (True, False):
+                    o = hw.Field(lat, src)
+                    D.hop(b, o, parity, sign, set_)
+                    bits.append(o.download())
+        for solve in (lambda x: hw.CG(D, accuracy=ACC, true_residual=True).apply(b, x),
+                      lambda x: hw.Hasenbusch_operator(D, 0.05).solve(b, x, accuracy=ACC),
+                      lambda x: D.solve(b, x, accuracy=ACC, use_graph=False)):
+            x = hw.Field(lat, guess)
+            r = solve(x)
+            assert r.converged and r.true_residual <= ACC
+            sols.append((r.iterations, x.download()))
+        return bits, sols
+
+    split, one = run(None), run("0")
+    for a, b in zip(split[0], one[0]):
+        assert np.array_equal(a, b)
+    for (ia, a), (ib, b) in zip(split[1], one[1]):
+        assert abs(ia - ib) <= 2 and rel(a, b) <= SOL_TOL
+
+
+def test_cg_limits(hw, ctx, oracle):
+    """A zero source, an iteration limit, and the same bits on a repeated solve."""
+    dims = (4, 4, 4, 4)
+    lat = hw.Lattice(ctx, dims)
+    D = hw.Dirac_Wilson_evenodd(0.12, hw.GaugeField(lat, oracle.gen_links(dims, 0.3, 5)))
+    zero, x = hw.Field(lat), hw.Field(lat)
+    r = hw.CG(D).apply(zero, x)
+    assert r.converged and r.iterations == 0 and not x.download().any()
+    b = hw.Field(lat, oracle.gen_spinor(dims, 6, oracle.EVEN))
+    r = D.solve(b, x, accuracy=1e-10, maxiters=3)
+    assert r.status == hw.HW_ERR_NOT_CONVERGED and r.iterations == 3
+    runs = []
+    for _ in range(2):
+        x.zero()
+        r = D.solve(b, x, accuracy=1e-10)
+        runs.append((r.iterations, x.download().tobytes()))
+    assert runs[0] == runs[1]

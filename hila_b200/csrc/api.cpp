@@ -494,6 +494,10 @@ CgWorkspace::~CgWorkspace() {
     if (loop_exec) cudaGraphExecDestroy(loop_exec);
 }
 
+LoopCgWorkspace::~LoopCgWorkspace() {
+    if (loop_exec) cudaGraphExecDestroy(loop_exec);
+}
+
 hw_lattice::~hw_lattice() {
     hw_field_destroy(host_b);
     hw_field_destroy(host_x);

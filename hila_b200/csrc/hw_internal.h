@@ -110,6 +110,23 @@ struct CgWorkspace {
     ~CgWorkspace();
 };
 
+// Workspace of a CG over device fields that keeps its loop graph (solver_full.cu,
+// staggered.cu): the iterated fields and the solution are the workspace's own, so the graph
+// serves every source and solution on the lattice.
+struct LoopCgWorkspace {
+    hw::DevBuf r[2], p[2], Dp[2], x[2], t;  // [0] EVEN, [1] ODD (unpreconditioned solve only)
+    cudaGraphExec_t loop_exec = nullptr;
+    struct Key {
+        const void *links = nullptr, *red = nullptr;
+        int planes = 0;
+        double par = 0;  // kappa or mass
+        bool operator==(const Key &o) const {
+            return links == o.links && red == o.red && planes == o.planes && par == o.par;
+        }
+    } key;
+    ~LoopCgWorkspace();
+};
+
 struct hw_field;
 
 struct hw_lattice {
@@ -120,6 +137,7 @@ struct hw_lattice {
     int stride = 0;
     hw::Geom g{};
     std::unique_ptr<CgWorkspace> ws;
+    std::unique_ptr<LoopCgWorkspace> full_ws, stag_ws;  // unpreconditioned and staggered CG
     hw_field *host_b = nullptr, *host_x = nullptr;  // fields behind the host-array solve
     bool tuned = false;  // FP64 hop launch shape chosen (g.hop_variant)
     ~hw_lattice();
@@ -148,6 +166,10 @@ struct hw_stag_field {
 namespace hw {
 int ensure_workspace(hw_lattice *lat);
 int ensure_reduction_capacity(hw_context *ctx, long nblocks);
+// Loop graph of a CG: WHILE(status == running) { body }, where body enqueues one iteration on
+// the stream and its last kernel sets the handle it is given (loop_next); replaces *exec
+template <class Body>
+int build_loop_graph(cudaStream_t s, cudaGraphExec_t *exec, Body body);
 int ensure_stage(hw_context *ctx, size_t bytes);
 // pick the fastest FP64 hop launch shape for this lattice once (HW_HOP_VARIANT overrides)
 int tune_hop(hw_lattice *lat, const hw_gauge *G);
@@ -155,4 +177,29 @@ int tune_hop(hw_lattice *lat, const hw_gauge *G);
 // ODD workspace field; context lock held, workspace and hop shape ready
 void eo_apply_half(const hw_gauge *G, double kappa, HalfF64 in, HalfF64 out, int sign, double d);
 void destroy_engines(hw_context *ctx);
+
+template <class Body>
+int build_loop_graph(cudaStream_t s, cudaGraphExec_t *exec, Body body) {
+    if (*exec) cudaGraphExecDestroy(*exec);
+    *exec = nullptr;
+    cudaGraph_t g = nullptr;
+    HW_CUDA(cudaGraphCreate(&g, 0));
+    cudaGraphConditionalHandle cond;
+    HW_CUDA(cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault));
+    cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
+    np.conditional.handle = cond;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t wnode;
+    HW_CUDA(cudaGraphAddNode(&wnode, g, nullptr, 0, &np));
+    HW_CUDA(cudaStreamBeginCaptureToGraph(s, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                          cudaStreamCaptureModeThreadLocal));
+    body(cond);
+    cudaGraph_t captured = nullptr;
+    HW_CUDA(cudaStreamEndCapture(s, &captured));
+    const cudaError_t e = cudaGraphInstantiate(exec, g, 0);
+    cudaGraphDestroy(g);
+    HW_CUDA(e);
+    return HW_OK;
+}
 }  // namespace hw

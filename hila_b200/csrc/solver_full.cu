@@ -1,99 +1,208 @@
 // CG<Dirac_Wilson>::apply (libraries/dirac/conjugate_gradient.h:46-104 on the
 // unpreconditioned operator of wilson.h:146-201): M^dag M out = in on ALL sites, FP64.
 //
-// The unpreconditioned operator is the reference's test operator (test_CG.cpp:127-182),
-// not the production path, so this solver is a plain host loop over device kernels:
-// the operator (two fused hop launches per application), and dot products and axpys
-// over whole fields.  A field's two halves are contiguous plane arrays whose padding
-// sites are never written, so the vector kernels run over the flat arrays.  Partial
-// sums are added on the host in block order: the result does not depend on scheduling.
+// An iteration is three kernels resident on the device (the body of a
+// CUDA-graph WHILE node, as solver_f64.cpp): K1 Dp = D p with |Dp|^2 -> alpha, K2 r -= alpha
+// D^dag Dp, x += alpha p with |r|^2 -> beta and the stopping decision, both over the two
+// parities in one launch, and p = r + beta p.  (A host loop over the operator, dot products
+// and axpys, with two host synchronisations per iteration and its workspace allocated per
+// call, took 107 us per iteration at 16^4.)  Partial sums are added in block order: the
+// result does not depend on scheduling.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <vector>
 
 #include "hw_internal.h"
 #include "reduce.cuh"
+#include "storage.cuh"
 
 namespace hw {
 namespace {
 
-constexpr int kFlatBlock = 256;
-constexpr int kFlatMaxBlocks = 1024;
-
-// partials[block] = sum Re conj(a) b over the block's elements of both halves
-__global__ void __launch_bounds__(kFlatBlock) k_flat_dot(long n, const double2 *a0, const double2 *b0,
-                                                         const double2 *a1, const double2 *b1, double *partials) {
-    __shared__ double smem[kFlatBlock / 32];
-    double s = 0.0;
-    for (long k = blockIdx.x * (long)kFlatBlock + threadIdx.x; k < n; k += (long)gridDim.x * kFlatBlock) {
-        const double2 x0 = a0[k], y0 = b0[k], x1 = a1[k], y1 = b1[k];
-        s += x0.x * y0.x + x0.y * y0.y + x1.x * y1.x + x1.y * y1.y;
-    }
-    const double t = block_sum<kFlatBlock>(s, smem);
-    if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-
-// y = a x + b y over both halves
-__global__ void __launch_bounds__(kFlatBlock) k_flat_axpby(long n, double a, const double2 *x0, const double2 *x1,
-                                                           double b, double2 *y0, double2 *y1) {
-    for (long k = blockIdx.x * (long)kFlatBlock + threadIdx.x; k < n; k += (long)gridDim.x * kFlatBlock) {
-        const double2 u0 = x0[k], u1 = x1[k];
-        double2 v0 = y0[k], v1 = y1[k];
-        v0.x = a * u0.x + b * v0.x;
-        v0.y = a * u0.y + b * v0.y;
-        v1.x = a * u1.x + b * v1.x;
-        v1.y = a * u1.y + b * v1.y;
-        y0[k] = v0;
-        y1[k] = v1;
-    }
-}
+constexpr int kFullBlock = 128;
 
 struct Full {  // the two halves of a Wilson field
     double2 *h[2];
 };
 
-class FullVec {
-  public:
-    int init(hw_lattice *lat) {
-        ctx_ = lat->ctx;
-        n_ = (long)12 * lat->stride;
-        blocks_ = (int)std::min<long>((n_ + kFlatBlock - 1) / kFlatBlock, kFlatMaxBlocks);
-        host_.resize(blocks_);
-        return partials_.alloc(sizeof(double) * blocks_);
-    }
-    int dot(Full a, Full b, double *out) {
-        k_flat_dot<<<blocks_, kFlatBlock, 0, ctx_->stream>>>(n_, a.h[0], b.h[0], a.h[1], b.h[1],
-                                                              partials_.as<double>());
-        HW_CUDA(cudaGetLastError());
-        HW_CUDA(cudaMemcpyAsync(host_.data(), partials_.ptr, sizeof(double) * blocks_, cudaMemcpyDeviceToHost,
-                                ctx_->stream));
-        HW_CUDA(cudaStreamSynchronize(ctx_->stream));
-        double s = 0.0;
-        for (int k = 0; k < blocks_; k++) s += host_[k];
-        *out = s;
-        return HW_OK;
-    }
-    int axpby(double a, Full x, double b, Full y) {
-        k_flat_axpby<<<blocks_, kFlatBlock, 0, ctx_->stream>>>(n_, a, x.h[0], x.h[1], b, y.h[0], y.h[1]);
-        HW_CUDA(cudaGetLastError());
-        return HW_OK;
-    }
-    int copy(Full src, Full dst) {
-        for (int p = 0; p < 2; p++)
-            HW_CUDA(cudaMemcpyAsync(dst.h[p], src.h[p], n_ * sizeof(double2), cudaMemcpyDeviceToDevice,
-                                    ctx_->stream));
-        return HW_OK;
-    }
+__device__ __forceinline__ Cx<double> ldf(const Full &f, int par, int stride, int c, int i) {
+    const double2 v = f.h[par][(size_t)c * stride + i];
+    return {v.x, v.y};
+}
+__device__ __forceinline__ void stf(const Full &f, int par, int stride, int c, int i, Cx<double> v) {
+    f.h[par][(size_t)c * stride + i] = make_double2(v.re, v.im);
+}
 
-  private:
-    hw_context *ctx_ = nullptr;
-    long n_ = 0;
-    int blocks_ = 1;
-    DevBuf partials_;
-    std::vector<double> host_;
+// out = in - k H in; ALPHA: |out|^2 -> alpha
+template <bool ALPHA>
+struct FullMul {
+    static constexpr int NRED = ALPHA ? 1 : 0;
+    Full in, out;
+    double k;
+    CgState *st;
+    __device__ bool skip() const { return ALPHA && st->status != CG_RUNNING; }
+    __device__ void operator()(int par, int stride, int i, const Spinor<double> &acc, double *red) const {
+        double n2 = 0;
+#pragma unroll
+        for (int c = 0; c < 12; c++) {
+            const Cx<double> v = ldf(in, par, stride, c, i) - k * acc.s[c / 3][c % 3];
+            stf(out, par, stride, c, i, v);
+            n2 += norm2(v);
+        }
+        red[0] = n2;
+    }
+    __device__ void operator()(const double *tot) {
+        st->pAp = tot[0];
+        if (!(tot[0] > 0.0) || !isfinite(tot[0]))
+            st->status = CG_BREAKDOWN, st->do_pupdate = 0;
+        else
+            st->alpha = st->rr / tot[0];
+    }
 };
+
+// the status after |r|^2 = rr, as conjugate_gradient.h:66-69 loops: while rr >= target
+__device__ __forceinline__ void full_status(CgState *st) {
+    if (!(st->rr >= st->target_rr))
+        st->status = CG_CONVERGED;
+    else if (st->iter >= st->maxiter)
+        st->status = CG_MAXITER;
+    else
+        st->status = CG_RUNNING;
+}
+
+// r = p = b - (Dp - k H Dp); |r|^2, |b|^2 -> the start of the iteration
+struct FullInit {
+    static constexpr int NRED = 2;
+    Full Dp, b, r, p;
+    double k, acc2;
+    int maxiter;
+    CgState *st;
+    __device__ bool skip() const { return false; }
+    __device__ void operator()(int par, int stride, int i, const Spinor<double> &acc, double *red) const {
+#pragma unroll
+        for (int c = 0; c < 12; c++) {
+            const Cx<double> bv = ldf(b, par, stride, c, i);
+            const Cx<double> v = bv - (ldf(Dp, par, stride, c, i) - k * acc.s[c / 3][c % 3]);
+            stf(r, par, stride, c, i, v);
+            stf(p, par, stride, c, i, v);
+            red[0] += norm2(v);
+            red[1] += norm2(bv);
+        }
+    }
+    __device__ void operator()(const double *tot) {
+        st->rr = tot[0];
+        st->src_norm2 = tot[1];
+        st->target_rr = acc2 * tot[1];
+        st->iter = 0;
+        st->maxiter = maxiter;
+        st->alpha = st->beta = 0.0;
+        st->do_pupdate = 0;
+        full_status(st);
+        if (!(tot[1] > 0.0)) st->status = CG_CONVERGED;
+    }
+};
+
+// r -= alpha (Dp - k H Dp), x += alpha p; |r|^2 -> beta, status
+struct FullUpdate {
+    static constexpr int NRED = 1;
+    Full Dp, r, x, p;
+    double k;
+    CgState *st;
+    __device__ bool skip() const { return st->status != CG_RUNNING; }
+    __device__ void operator()(int par, int stride, int i, const Spinor<double> &acc, double *red) const {
+        const double alpha = st->alpha;
+        double n2 = 0;
+#pragma unroll
+        for (int c = 0; c < 12; c++) {
+            const Cx<double> ddp = ldf(Dp, par, stride, c, i) - k * acc.s[c / 3][c % 3];
+            const Cx<double> rv = ldf(r, par, stride, c, i) - alpha * ddp;
+            stf(r, par, stride, c, i, rv);
+            stf(x, par, stride, c, i, ldf(x, par, stride, c, i) + alpha * ldf(p, par, stride, c, i));
+            n2 += norm2(rv);
+        }
+        red[0] = n2;
+    }
+    __device__ void operator()(const double *tot) {
+        st->iter += 1;
+        st->beta = tot[0] / st->rr;
+        st->rr = tot[0];
+        st->do_pupdate = 1;
+        full_status(st);
+    }
+};
+
+// |b - (Dp - k H Dp)|^2
+struct FullResidual {
+    static constexpr int NRED = 1;
+    Full Dp, b;
+    double k;
+    CgState *st;
+    __device__ bool skip() const { return false; }
+    __device__ void operator()(int par, int stride, int i, const Spinor<double> &acc, double *red) const {
+#pragma unroll
+        for (int c = 0; c < 12; c++)
+            red[0] += norm2(ldf(b, par, stride, c, i) - (ldf(Dp, par, stride, c, i) - k * acc.s[c / 3][c % 3]));
+    }
+    __device__ void operator()(const double *tot) { st->res_num2 = tot[0]; }
+};
+
+// the hop over both parities: blocks [0, n) EVEN output sites, [n, 2n) ODD ones
+template <int SIGN, class Lk, class Epi>
+__global__ void __launch_bounds__(kFullBlock, 4) k_full_hop(Geom g, Lk U, Full in, Epi epi, RedBuf red) {
+    if (epi.skip()) return;
+    const int nb = gridDim.x / 2;
+    const int par = (int)blockIdx.x >= nb ? 1 : 0;
+    const int i = ((int)blockIdx.x - par * nb) * kFullBlock + threadIdx.x;
+    constexpr int NR = Epi::NRED > 0 ? Epi::NRED : 1;
+    double v[NR];
+#pragma unroll
+    for (int k = 0; k < NR; k++) v[k] = 0.0;
+    if (i < g.Vh) {
+        Spinor<double> acc;
+        hop_site<SIGN>(g, par, i, SpinorF64{in.h[1 - par], U.stride}, U, acc);
+        epi(par, U.stride, i, acc, v);
+    }
+    if constexpr (Epi::NRED > 0) grid_reduce<Epi::NRED, kFullBlock>(v, red.partials, red.ticket, epi);
+}
+
+// p = r + beta p over both halves
+__global__ void __launch_bounds__(256) k_full_pupdate(long n, Full r, Full p, const CgState *st,
+                                                     cudaGraphConditionalHandle cond) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) loop_next(st, cond, 1);
+    if (!st->do_pupdate) return;
+    const double beta = st->beta;
+    const long k = blockIdx.x * 256L + threadIdx.x;
+    if (k >= n) return;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const double2 rv = r.h[h][k], pv = p.h[h][k];
+        p.h[h][k] = make_double2(fma(beta, pv.x, rv.x), fma(beta, pv.y, rv.y));
+    }
+}
+
+template <class Epi>
+void full_hop(const hw_gauge *G, int sign, Full in, const Epi &epi, RedBuf red, cudaStream_t s) {
+    const Geom &g = G->lat->g;
+    const GaugeF64 U = G->U();
+    const int nb = 2 * ((g.Vh + kFullBlock - 1) / kFullBlock);
+    const LinksF64x18 U18{U.p, U.stride};
+    const LinksF64x12 U12{U.p, U.stride};
+    if (U.planes == 9) {
+        if (sign > 0)
+            k_full_hop<1><<<nb, kFullBlock, 0, s>>>(g, U18, in, epi, red);
+        else
+            k_full_hop<-1><<<nb, kFullBlock, 0, s>>>(g, U18, in, epi, red);
+    } else {
+        if (sign > 0)
+            k_full_hop<1><<<nb, kFullBlock, 0, s>>>(g, U12, in, epi, red);
+        else
+            k_full_hop<-1><<<nb, kFullBlock, 0, s>>>(g, U12, in, epi, red);
+    }
+}
+
+Full full_of(const DevBuf (&b)[2]) { return Full{{b[0].as<double2>(), b[1].as<double2>()}}; }
 
 Full full_of(const hw_field *f) { return Full{{f->half[0].buf.as<double2>(), f->half[1].buf.as<double2>()}}; }
 
@@ -117,80 +226,69 @@ extern "C" int hw_wilson_cg_solve(const hw_gauge *gauge, double kappa, const hw_
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     HW_CUDA(cudaSetDevice(ctx->device));
     int rc;
-    // workspace fields r, p, A p and the intermediate M v
-    hw_field *ws[4] = {nullptr, nullptr, nullptr, nullptr};
-    auto release = [&]() {
-        for (hw_field *f : ws) hw_field_destroy(f);
-    };
-    for (hw_field *&f : ws)
-        if ((rc = hw_field_create(lat, &f)) != HW_OK) {
-            release();
-            return rc;
-        }
-    FullVec V;
-    if ((rc = V.init(lat)) != HW_OK) {
-        release();
-        return rc;
+    if ((rc = ensure_reduction_capacity(ctx, 2 * ((lat->Vh + kFullBlock - 1) / kFullBlock))) != HW_OK) return rc;
+    if (!lat->full_ws) lat->full_ws.reset(new LoopCgWorkspace());
+    LoopCgWorkspace &w = *lat->full_ws;
+    const size_t hb = (size_t)12 * lat->stride * sizeof(double2);
+    cudaStream_t s = ctx->stream;
+    for (int h = 0; h < 2; h++)
+        for (DevBuf *d : {&w.r[h], &w.p[h], &w.Dp[h], &w.x[h]})
+            if (!d->ptr) {
+                if ((rc = d->alloc(hb)) != HW_OK) return rc;
+                HW_CUDA(cudaMemsetAsync(d->ptr, 0, hb, s));  // the padding sites of p are read by its update
+            }
+    const Full b = full_of(in), xo = full_of(out), x = full_of(w.x), r = full_of(w.r), p = full_of(w.p),
+               Dp = full_of(w.Dp);
+    CgState *st = ctx->cg_state.as<CgState>();
+    const RedBuf red = ctx->red();
+    const long n = (long)12 * lat->stride;
+    LoopCgWorkspace::Key key;
+    key.links = gauge->U().p;
+    key.planes = gauge->U().planes;
+    key.red = red.partials;
+    key.par = kappa;
+    if (!w.loop_exec || !(key == w.key)) {
+        w.key = LoopCgWorkspace::Key();
+        rc = build_loop_graph(s, &w.loop_exec, [&](cudaGraphConditionalHandle cond) {
+            full_hop(gauge, 1, p, FullMul<true>{p, Dp, kappa, st}, red, s);
+            full_hop(gauge, -1, Dp, FullUpdate{Dp, r, x, p, kappa, st}, red, s);
+            k_full_pupdate<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, r, p, st, cond);
+        });
+        if (rc != HW_OK) return rc;
+        w.key = key;
     }
-    const Full b = full_of(in), x = full_of(out), r = full_of(ws[0]), p = full_of(ws[1]), Ap = full_of(ws[2]);
-    auto A = [&](const hw_field *v, hw_field *w) {  // w = M^dag M v
-        int e = hw_wilson_apply(gauge, kappa, 1, v, ws[3]);
-        return e != HW_OK ? e : hw_wilson_apply(gauge, kappa, -1, ws[3], w);
-    };
-    auto body = [&](hw_cg_result *R) -> int {
-        cudaStream_t s = ctx->stream;
-        HW_CUDA(cudaEventRecord(ctx->ev0, s));
-        int e;
-        // r = b - A x ; p = r   (conjugate_gradient.h:57-63)
-        if ((e = A(out, ws[2])) != HW_OK) return e;
-        if ((e = V.copy(b, r)) != HW_OK || (e = V.axpby(-1.0, Ap, 1.0, r)) != HW_OK || (e = V.copy(r, p)) != HW_OK)
-            return e;
-        double bb, rr;
-        if ((e = V.dot(b, b, &bb)) != HW_OK || (e = V.dot(r, r, &rr)) != HW_OK) return e;
-        const double target = P.accuracy * P.accuracy * bb;
-        int it = 0, status = HW_OK;
-        while (rr >= target && bb > 0) {
-            if (it >= P.maxiters) {
-                status = HW_ERR_NOT_CONVERGED;
-                break;
-            }
-            if ((e = A(ws[1], ws[2])) != HW_OK) return e;
-            double pAp;
-            if ((e = V.dot(p, Ap, &pAp)) != HW_OK) return e;
-            if (!(pAp > 0.0) || !std::isfinite(pAp)) {
-                status = HW_ERR_BREAKDOWN;
-                break;
-            }
-            const double alpha = rr / pAp;
-            if ((e = V.axpby(alpha, p, 1.0, x)) != HW_OK || (e = V.axpby(-alpha, Ap, 1.0, r)) != HW_OK) return e;
-            double rr_new;
-            if ((e = V.dot(r, r, &rr_new)) != HW_OK) return e;
-            const double beta = rr_new / rr;
-            rr = rr_new;
-            if ((e = V.axpby(1.0, r, beta, p)) != HW_OK) return e;
-            it++;
-        }
-        // explicit residual |b - A x| / |b| in FP64
-        if ((e = A(out, ws[2])) != HW_OK) return e;
-        if ((e = V.copy(b, r)) != HW_OK || (e = V.axpby(-1.0, Ap, 1.0, r)) != HW_OK) return e;
-        double res2;
-        if ((e = V.dot(r, r, &res2)) != HW_OK) return e;
-        HW_CUDA(cudaEventRecord(ctx->ev1, s));
-        HW_CUDA(cudaEventSynchronize(ctx->ev1));
-        const double true_res = bb > 0 ? std::sqrt(res2 / bb) : 0.0;
-        if (status == HW_OK && P.true_residual && true_res > P.accuracy) status = HW_ERR_NOT_CONVERGED;
-        std::memset(R, 0, sizeof(*R));
+    HW_CUDA(cudaEventRecord(ctx->ev0, s));
+    for (int h = 0; h < 2; h++) HW_CUDA(cudaMemcpyAsync(x.h[h], xo.h[h], hb, cudaMemcpyDeviceToDevice, s));
+    // r = b - A x ; p = r   (conjugate_gradient.h:57-63)
+    full_hop(gauge, 1, x, FullMul<false>{x, Dp, kappa, st}, red, s);
+    full_hop(gauge, -1, Dp, FullInit{Dp, b, r, p, kappa, P.accuracy * P.accuracy, P.maxiters, st}, red, s);
+    HW_CUDA(cudaGetLastError());
+    HW_CUDA(cudaGraphLaunch(w.loop_exec, s));
+    // explicit residual |b - A x| in FP64
+    full_hop(gauge, 1, x, FullMul<false>{x, Dp, kappa, st}, red, s);
+    full_hop(gauge, -1, Dp, FullResidual{Dp, b, kappa, st}, red, s);
+    for (int h = 0; h < 2; h++) HW_CUDA(cudaMemcpyAsync(xo.h[h], x.h[h], hb, cudaMemcpyDeviceToDevice, s));
+    HW_CUDA(cudaGetLastError());
+    HW_CUDA(cudaEventRecord(ctx->ev1, s));
+    CgState *h = ctx->cg_state_host;
+    HW_CUDA(cudaMemcpyAsync(h, st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
+    HW_CUDA(cudaStreamSynchronize(s));
+    const double bb = h->src_norm2;
+    const double true_res = bb > 0 ? std::sqrt(h->res_num2 / bb) : 0.0;
+    int status = h->status == CG_BREAKDOWN ? HW_ERR_BREAKDOWN
+                 : h->status == CG_MAXITER ? HW_ERR_NOT_CONVERGED
+                                           : HW_OK;
+    if (status == HW_OK && P.true_residual && true_res > P.accuracy) status = HW_ERR_NOT_CONVERGED;
+    if (result) {
+        std::memset(result, 0, sizeof(*result));
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-        R->status = status;
-        R->iterations = it;
-        R->rr_relative = bb > 0 ? rr / bb : 0.0;
-        R->true_residual = true_res;
-        R->seconds = ms * 1e-3;
-        return status;
-    };
-    hw_cg_result tmp;
-    rc = body(result ? result : &tmp);
-    release();
-    return rc;
+        result->status = status;
+        result->iterations = h->iter;
+        result->rr_relative = bb > 0 ? h->rr / bb : 0.0;
+        result->true_residual = true_res;
+        result->seconds = ms * 1e-3;
+        result->kernel_launches = 4 + 3 * std::max(h->iter, 1);
+    }
+    return status;
 }

@@ -10,9 +10,9 @@
 // half lattices of 3 double2 planes (stride = the lattice's padded parity size).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <vector>
 
 #include "hw_internal.h"
 #include "reduce.cuh"
@@ -25,7 +25,6 @@ namespace {
 
 constexpr int kStagBlock = 128;
 constexpr int kStagVecBlock = 256;
-constexpr int kStagMaxBlocks = 1024;
 
 HalfStag half_of(const hw_stag_field *f, int p) {
     return HalfStag{f->half[p].as<double2>(), f->lat->stride};
@@ -90,61 +89,186 @@ __global__ void k_stag_layout(Geom g, int par, double2 *lex, HalfStag f, int to_
     }
 }
 
-// ---- vector operations on EVEN halves (deterministic partial sums, summed on the host in order)
-__global__ void __launch_bounds__(kStagVecBlock) k_stag_dot(int Vh, HalfStag a, HalfStag b, double *partials) {
-    __shared__ double smem[kStagVecBlock / 32];
-    double s = 0.0;
-    for (int i = blockIdx.x * kStagVecBlock + threadIdx.x; i < Vh; i += gridDim.x * kStagVecBlock)
+// ---- CG on the normal equations, resident on the device (the body of a CUDA-graph WHILE
+// node, as solver_f64.cpp): t = (1/m) D p, Dp = m p + D t with |Dp|^2 -> alpha, t = (1/m)
+// D^dag Dp, then r -= alpha M^dag Dp, x += alpha p with |r|^2 -> beta and the stopping
+// decision, and p = r + beta p.  (A host loop over the operator, dot products and axpys with
+// two host synchronisations per iteration and its workspace allocated per call took 98 us
+// per iteration at 14x18x12x26.)  Partial sums are added in block order.
+
+// t = a 0.5 s hop in
+struct StagScale {
+    static constexpr int NRED = 0;
+    HalfStag out;
+    double a;
+    const CgState *st;
+    __device__ bool skip() const { return st && st->status != CG_RUNNING; }
+    __device__ void operator()(int i, const Cx<double> (&h)[3], double *) const {
+#pragma unroll
+        for (int k = 0; k < 3; k++) out.st(k, i, a * h[k]);
+    }
+    __device__ void operator()(const double *) const {}
+};
+
+// Dp = m p + h; ALPHA: |Dp|^2 -> alpha
+template <bool ALPHA>
+struct StagMul {
+    static constexpr int NRED = ALPHA ? 1 : 0;
+    HalfStag p, Dp;
+    double m;
+    CgState *st;
+    __device__ bool skip() const { return ALPHA && st->status != CG_RUNNING; }
+    __device__ void operator()(int i, const Cx<double> (&h)[3], double *red) const {
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            const double2 u = a.p[(size_t)k * a.stride + i], v = b.p[(size_t)k * b.stride + i];
-            s += u.x * v.x + u.y * v.y;
+            const Cx<double> v = m * p.ldp(k, i) + h[k];
+            Dp.st(k, i, v);
+            red[0] += norm2(v);
         }
-    const double t = block_sum<kStagVecBlock>(s, smem);
-    if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-
-// y = a x + b y (x may alias nothing; b = 1 gives axpy)
-__global__ void __launch_bounds__(kStagVecBlock) k_stag_axpby(int Vh, double a, HalfStag x, double b, HalfStag y) {
-    for (int i = blockIdx.x * kStagVecBlock + threadIdx.x; i < Vh; i += gridDim.x * kStagVecBlock)
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const double2 u = x.p[(size_t)k * x.stride + i];
-            double2 &v = y.p[(size_t)k * y.stride + i];
-            v = make_double2(a * u.x + b * v.x, a * u.y + b * v.y);
-        }
-}
-
-struct StagVec {
-    hw_context *ctx;
-    int Vh, blocks;
-    DevBuf partials;
-    std::vector<double> host;
-    int init(hw_lattice *lat) {
-        ctx = lat->ctx;
-        Vh = (int)lat->Vh;
-        blocks = (int)std::min<long>((lat->Vh + kStagVecBlock - 1) / kStagVecBlock, kStagMaxBlocks);
-        host.resize(blocks);
-        return partials.alloc(sizeof(double) * blocks);
     }
-    // Re <a, b> over EVEN
-    int dot(HalfStag a, HalfStag b, double *out) {
-        k_stag_dot<<<blocks, kStagVecBlock, 0, ctx->stream>>>(Vh, a, b, partials.as<double>());
-        HW_CUDA(cudaGetLastError());
-        HW_CUDA(cudaMemcpyAsync(host.data(), partials.ptr, sizeof(double) * blocks, cudaMemcpyDeviceToHost,
-                                ctx->stream));
-        HW_CUDA(cudaStreamSynchronize(ctx->stream));
-        double s = 0.0;
-        for (int k = 0; k < blocks; k++) s += host[k];
-        *out = s;
-        return HW_OK;
-    }
-    int axpby(double a, HalfStag x, double b, HalfStag y) {
-        k_stag_axpby<<<blocks, kStagVecBlock, 0, ctx->stream>>>(Vh, a, x, b, y);
-        HW_CUDA(cudaGetLastError());
-        return HW_OK;
+    __device__ void operator()(const double *tot) const {
+        st->pAp = tot[0];
+        if (!(tot[0] > 0.0) || !isfinite(tot[0]))
+            st->status = CG_BREAKDOWN, st->do_pupdate = 0;
+        else
+            st->alpha = st->rr / tot[0];
     }
 };
+
+// the status after |r|^2 = rr, as conjugate_gradient.h:66-69 loops: while rr >= target
+__device__ __forceinline__ void stag_status(CgState *st) {
+    if (!(st->rr >= st->target_rr))
+        st->status = CG_CONVERGED;
+    else if (st->iter >= st->maxiter)
+        st->status = CG_MAXITER;
+    else
+        st->status = CG_RUNNING;
+}
+
+// r = p = b - (m Dp + h); |r|^2, |b|^2 -> the start of the iteration
+struct StagInit {
+    static constexpr int NRED = 2;
+    HalfStag Dp, b, r, p;
+    double m, acc2;
+    int maxiter;
+    CgState *st;
+    __device__ bool skip() const { return false; }
+    __device__ void operator()(int i, const Cx<double> (&h)[3], double *red) const {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const Cx<double> bv = b.ldp(k, i);
+            const Cx<double> v = bv - (m * Dp.ldp(k, i) + h[k]);
+            r.st(k, i, v);
+            p.st(k, i, v);
+            red[0] += norm2(v);
+            red[1] += norm2(bv);
+        }
+    }
+    __device__ void operator()(const double *tot) const {
+        st->rr = tot[0];
+        st->src_norm2 = tot[1];
+        st->target_rr = acc2 * tot[1];
+        st->iter = 0;
+        st->maxiter = maxiter;
+        st->alpha = st->beta = 0.0;
+        st->do_pupdate = 0;
+        stag_status(st);
+        if (!(tot[1] > 0.0)) st->status = CG_CONVERGED;
+    }
+};
+
+// r -= alpha (m Dp + h), x += alpha p; |r|^2 -> beta, status
+struct StagUpdate {
+    static constexpr int NRED = 1;
+    HalfStag Dp, r, x, p;
+    double m;
+    CgState *st;
+    __device__ bool skip() const { return st->status != CG_RUNNING; }
+    __device__ void operator()(int i, const Cx<double> (&h)[3], double *red) const {
+        const double alpha = st->alpha;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const Cx<double> rv = r.ldp(k, i) - alpha * (m * Dp.ldp(k, i) + h[k]);
+            r.st(k, i, rv);
+            x.st(k, i, x.ldp(k, i) + alpha * p.ldp(k, i));
+            red[0] += norm2(rv);
+        }
+    }
+    __device__ void operator()(const double *tot) const {
+        st->iter += 1;
+        st->beta = tot[0] / st->rr;
+        st->rr = tot[0];
+        st->do_pupdate = 1;
+        stag_status(st);
+    }
+};
+
+// |b - (m Dp + h)|^2
+struct StagResidual {
+    static constexpr int NRED = 1;
+    HalfStag Dp, b;
+    double m;
+    CgState *st;
+    __device__ bool skip() const { return false; }
+    __device__ void operator()(int i, const Cx<double> (&h)[3], double *red) const {
+#pragma unroll
+        for (int k = 0; k < 3; k++) red[0] += norm2(b.ldp(k, i) - (m * Dp.ldp(k, i) + h[k]));
+    }
+    __device__ void operator()(const double *tot) const { st->res_num2 = tot[0]; }
+};
+
+template <int SIGN, class Lk, class Epi>
+__global__ void __launch_bounds__(kStagBlock) k_stag_cg(Geom g, Lk U, int par, HalfStag in, Epi epi, RedBuf red) {
+    if (epi.skip()) return;
+    const int i = blockIdx.x * kStagBlock + threadIdx.x;
+    constexpr int NR = Epi::NRED > 0 ? Epi::NRED : 1;
+    double v[NR];
+#pragma unroll
+    for (int k = 0; k < NR; k++) v[k] = 0.0;
+    if (i < g.Vh) {
+        Cx<double> acc[3];
+        stag_hop_site(g, U, par, i, in, acc);
+#pragma unroll
+        for (int k = 0; k < 3; k++) acc[k] = (0.5 * SIGN) * acc[k];
+        epi(i, acc, v);
+    }
+    if constexpr (Epi::NRED > 0) grid_reduce<Epi::NRED, kStagBlock>(v, red.partials, red.ticket, epi);
+}
+
+// p = r + beta p
+__global__ void __launch_bounds__(kStagVecBlock) k_stag_pupdate(int Vh, HalfStag r, HalfStag p, const CgState *st,
+                                                               cudaGraphConditionalHandle cond) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) loop_next(st, cond, 1);
+    if (!st->do_pupdate) return;
+    const int i = blockIdx.x * kStagVecBlock + threadIdx.x;
+    if (i >= Vh) return;
+    const double beta = st->beta;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const Cx<double> rv = r.ldp(k, i), pv = p.ldp(k, i);
+        p.st(k, i, {fma(beta, pv.re, rv.re), fma(beta, pv.im, rv.im)});
+    }
+}
+
+template <class Epi>
+void stag_cg(const hw_gauge *G, int par, int sign, HalfStag in, const Epi &epi, RedBuf red, cudaStream_t s) {
+    const GaugeF64 U = G->U();
+    const Geom &g = G->lat->g;
+    const int nb = (g.Vh + kStagBlock - 1) / kStagBlock;
+    const LinksF64x18 U18{U.p, U.stride};
+    const LinksF64x12 U12{U.p, U.stride};
+    if (U.planes == 9) {
+        if (sign > 0)
+            k_stag_cg<1><<<nb, kStagBlock, 0, s>>>(g, U18, par, in, epi, red);
+        else
+            k_stag_cg<-1><<<nb, kStagBlock, 0, s>>>(g, U18, par, in, epi, red);
+    } else {
+        if (sign > 0)
+            k_stag_cg<1><<<nb, kStagBlock, 0, s>>>(g, U12, par, in, epi, red);
+        else
+            k_stag_cg<-1><<<nb, kStagBlock, 0, s>>>(g, U12, par, in, epi, red);
+    }
+}
 
 // ---- force (staggered.h:70-86, 246-265); t1 = (1/m) hop_{-s} chi, t2 = (1/m) hop_s psi on ODD
 //   x even: F_d = -s/2 eta_d t1(x+d) (x) psi(x) + s/2 eta_d t2(x+d) (x) chi(x)
@@ -191,6 +315,16 @@ int check_stag_op(const hw_gauge *G, const hw_stag_field *a, const hw_stag_field
     HW_CHECK_ARG(G && a && b, "null argument");
     HW_CHECK_ARG(a->lat == G->lat && b->lat == G->lat, "fields and gauge live on different lattices");
     HW_CHECK_ARG(std::isfinite(mass) && mass != 0.0, "mass must be finite and non-zero");
+    return HW_OK;
+}
+
+// the lattice's staggered workspace (five half-lattice fields), kept with the lattice
+int ensure_stag_ws(hw_lattice *lat) {
+    if (!lat->stag_ws) lat->stag_ws.reset(new LoopCgWorkspace());
+    LoopCgWorkspace &w = *lat->stag_ws;
+    int rc;
+    for (DevBuf *d : {&w.r[0], &w.p[0], &w.Dp[0], &w.x[0], &w.t})
+        if (!d->ptr && (rc = d->alloc((size_t)3 * lat->stride * sizeof(double2))) != HW_OK) return rc;
     return HW_OK;
 }
 
@@ -333,7 +467,7 @@ int hw_staggered_evenodd_force(const hw_gauge *gauge, double mass, const hw_stag
 
 // CG<dirac_staggered_evenodd>::apply (conjugate_gradient.h:46-104): M^dag M out = in
 // on EVEN, out the initial guess; stops when |r|^2 < accuracy^2 |in|^2 (with
-// true_residual set, also on the recomputed |in - M^dag M out|).  FP64, host loop.
+// true_residual set, also on the recomputed |in - M^dag M out|).  FP64.
 int hw_staggered_cg_solve(const hw_gauge *gauge, double mass, const hw_stag_field *in, hw_stag_field *out,
                           const hw_cg_params *params, hw_cg_result *result) {
     int rc = check_stag_op(gauge, in, out, mass);
@@ -348,77 +482,74 @@ int hw_staggered_cg_solve(const hw_gauge *gauge, double mass, const hw_stag_fiel
     hw_context *ctx = lat->ctx;
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     HW_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = ensure_reduction_capacity(ctx, (lat->Vh + kStagBlock - 1) / kStagBlock)) != HW_OK) return rc;
+    if ((rc = ensure_stag_ws(lat)) != HW_OK) return rc;
+    LoopCgWorkspace &w = *lat->stag_ws;
     const int stride = lat->stride;
     const size_t hb = (size_t)3 * stride * sizeof(double2);
-    DevBuf br, bp, bAp, be, bo;
-    for (DevBuf *d : {&br, &bp, &bAp, &be, &bo})
-        if ((rc = d->alloc(hb)) != HW_OK) return rc;
-    const HalfStag r{br.as<double2>(), stride}, p{bp.as<double2>(), stride}, Ap{bAp.as<double2>(), stride};
-    const HalfStag te{be.as<double2>(), stride}, to{bo.as<double2>(), stride};
-    const HalfStag b = half_of(in, 0), x = half_of(out, 0);
-    StagVec V;
-    if ((rc = V.init(lat)) != HW_OK) return rc;
+    auto half = [stride](const DevBuf &d) { return HalfStag{d.as<double2>(), stride}; };
+    const HalfStag b = half_of(in, 0), xo = half_of(out, 0), x = half(w.x[0]), r = half(w.r[0]), p = half(w.p[0]),
+                   Dp = half(w.Dp[0]), t = half(w.t);
     cudaStream_t s = ctx->stream;
-    auto A = [&](HalfStag v, HalfStag w) {  // w = M^dag M v
-        stag_eo_apply(gauge, mass, v, te, to, +1, s);
-        stag_eo_apply(gauge, mass, te, w, to, -1, s);
+    CgState *st = ctx->cg_state.as<CgState>();
+    const RedBuf red = ctx->red();
+    const double im = 1.0 / mass;
+    LoopCgWorkspace::Key key;
+    key.links = gauge->U().p;
+    key.planes = gauge->U().planes;
+    key.red = red.partials;
+    key.par = mass;
+    if (!w.loop_exec || !(key == w.key)) {
+        w.key = LoopCgWorkspace::Key();
+        rc = build_loop_graph(s, &w.loop_exec, [&](cudaGraphConditionalHandle cond) {
+            stag_cg(gauge, 1, +1, p, StagScale{t, im, st}, red, s);
+            stag_cg(gauge, 0, +1, t, StagMul<true>{p, Dp, mass, st}, red, s);
+            stag_cg(gauge, 1, -1, Dp, StagScale{t, im, st}, red, s);
+            stag_cg(gauge, 0, -1, t, StagUpdate{Dp, r, x, p, mass, st}, red, s);
+            k_stag_pupdate<<<(unsigned)((lat->Vh + kStagVecBlock - 1) / kStagVecBlock), kStagVecBlock, 0, s>>>(
+                (int)lat->Vh, r, p, st, cond);
+        });
+        if (rc != HW_OK) return rc;
+        w.key = key;
+    }
+    // Dp = M x ; then the epilogue of M^dag Dp
+    auto normal = [&](auto epi) {
+        stag_cg(gauge, 1, +1, x, StagScale{t, im, nullptr}, red, s);
+        stag_cg(gauge, 0, +1, t, StagMul<false>{x, Dp, mass, st}, red, s);
+        stag_cg(gauge, 1, -1, Dp, StagScale{t, im, nullptr}, red, s);
+        stag_cg(gauge, 0, -1, t, epi, red, s);
     };
     HW_CUDA(cudaEventRecord(ctx->ev0, s));
+    HW_CUDA(cudaMemcpyAsync(x.p, xo.p, hb, cudaMemcpyDeviceToDevice, s));
     // r = b - A x ; p = r
-    A(x, Ap);
-    HW_CUDA(cudaMemcpyAsync(r.p, b.p, hb, cudaMemcpyDeviceToDevice, s));
-    if ((rc = V.axpby(-1.0, Ap, 1.0, r)) != HW_OK) return rc;
-    HW_CUDA(cudaMemcpyAsync(p.p, r.p, hb, cudaMemcpyDeviceToDevice, s));
-    double bb, rr;
-    if ((rc = V.dot(b, b, &bb)) != HW_OK) return rc;
-    if ((rc = V.dot(r, r, &rr)) != HW_OK) return rc;
-    const double target = P.accuracy * P.accuracy * bb;
-    int it = 0, status = HW_OK;
-    long launches = 4 + 2;
-    while (rr >= target && bb > 0) {
-        if (it >= P.maxiters) {
-            status = HW_ERR_NOT_CONVERGED;
-            break;
-        }
-        A(p, Ap);
-        double pAp;
-        if ((rc = V.dot(p, Ap, &pAp)) != HW_OK) return rc;
-        if (!(pAp > 0.0) || !std::isfinite(pAp)) {
-            status = HW_ERR_BREAKDOWN;
-            break;
-        }
-        const double alpha = rr / pAp;
-        if ((rc = V.axpby(alpha, p, 1.0, x)) != HW_OK) return rc;
-        if ((rc = V.axpby(-alpha, Ap, 1.0, r)) != HW_OK) return rc;
-        double rr_new;
-        if ((rc = V.dot(r, r, &rr_new)) != HW_OK) return rc;
-        const double beta = rr_new / rr;
-        rr = rr_new;
-        if ((rc = V.axpby(1.0, r, beta, p)) != HW_OK) return rc;
-        it++;
-        launches += 4 + 5;
-    }
+    normal(StagInit{Dp, b, r, p, mass, P.accuracy * P.accuracy, P.maxiters, st});
+    HW_CUDA(cudaGetLastError());
+    HW_CUDA(cudaGraphLaunch(w.loop_exec, s));
     // explicit residual |b - A x| / |b| in FP64
-    A(x, Ap);
-    HW_CUDA(cudaMemcpyAsync(r.p, b.p, hb, cudaMemcpyDeviceToDevice, s));
-    if ((rc = V.axpby(-1.0, Ap, 1.0, r)) != HW_OK) return rc;
-    double res2;
-    if ((rc = V.dot(r, r, &res2)) != HW_OK) return rc;
+    normal(StagResidual{Dp, b, mass, st});
+    HW_CUDA(cudaMemcpyAsync(xo.p, x.p, hb, cudaMemcpyDeviceToDevice, s));
     HW_CUDA(cudaMemsetAsync(out->half[1].ptr, 0, out->half[1].bytes, s));
+    HW_CUDA(cudaGetLastError());
     HW_CUDA(cudaEventRecord(ctx->ev1, s));
-    HW_CUDA(cudaEventSynchronize(ctx->ev1));
-    const double true_res = bb > 0 ? std::sqrt(res2 / bb) : 0.0;
+    CgState *h = ctx->cg_state_host;
+    HW_CUDA(cudaMemcpyAsync(h, st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
+    HW_CUDA(cudaStreamSynchronize(s));
+    const double bb = h->src_norm2;
+    const double true_res = bb > 0 ? std::sqrt(h->res_num2 / bb) : 0.0;
+    int status = h->status == CG_BREAKDOWN ? HW_ERR_BREAKDOWN
+                 : h->status == CG_MAXITER ? HW_ERR_NOT_CONVERGED
+                                           : HW_OK;
     if (status == HW_OK && P.true_residual && true_res > P.accuracy) status = HW_ERR_NOT_CONVERGED;
     if (result) {
         std::memset(result, 0, sizeof(*result));
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
         result->status = status;
-        result->iterations = it;
-        result->rr_relative = bb > 0 ? rr / bb : 0.0;
+        result->iterations = h->iter;
+        result->rr_relative = bb > 0 ? h->rr / bb : 0.0;
         result->true_residual = true_res;
         result->seconds = ms * 1e-3;
-        result->kernel_launches = (int)(launches + 6);
+        result->kernel_launches = 8 + 5 * std::max(h->iter, 1);
     }
     return status;
 }

@@ -81,3 +81,30 @@ def test_cg_limits(hw, ctx, oracle):
         r = D.solve(b, x, accuracy=1e-10)
         runs.append((r.iterations, x.download().tobytes()))
     assert runs[0] == runs[1]
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 2, 4, 10), (8, 8, 8, 8)])
+@pytest.mark.parametrize("link_format", [18, 12])
+def test_loop_graph_solvers(hw, ctx, oracle, dims, link_format):
+    """Several sources, solutions, couplings and gauge fields on one lattice share a workspace and
+    rebuild its loop graph; the operator of the solution gives the source back."""
+    lat = hw.Lattice(ctx, dims)
+    for seed, kappa, mass in ((5, 0.11, 4.0), (6, 0.11, 4.0), (6, 0.12, 5.0)):
+        G = hw.GaugeField(lat, oracle.gen_links(dims, 0.3, seed), link_format)
+        D, S = hw.Dirac_Wilson(kappa, G), hw.dirac_staggered_evenodd(mass, G)
+        for k in range(2):
+            b, x, y, z = (hw.Field(lat, oracle.gen_spinor(dims, 10 + k, oracle.ALL)), hw.Field(lat), hw.Field(lat),
+                          hw.Field(lat))
+            r = D.cg(b, x, accuracy=ACC)
+            assert r.converged
+            D.apply(x, y)
+            D.dagger(y, z)
+            assert rel(z.download(), b.download()) <= 10 * ACC
+            rng = np.random.default_rng(20 + k)
+            sb = hw.StaggeredField(lat, rng.standard_normal((lat.volume, 3, 2)), hw.EVEN)
+            sx, sy, sz = (hw.StaggeredField(lat) for _ in range(3))
+            r = S.cg(sb, sx, accuracy=ACC)
+            assert r.converged
+            S.apply(sx, sy)
+            S.dagger(sy, sz)
+            assert rel(sz.download(hw.EVEN), sb.download(hw.EVEN)) <= 10 * ACC

@@ -459,8 +459,13 @@ int Engine::configure() {
     const bool known =
         variant == 2 || (low_ == LOW_F16 && (variant == 7 || (variant == 4 && full18_)));
     if (!known) variant = default_variant();
-    if (variant != grid_.variant || mask != grid_.planes_mask || fermions != grid_.fermions) {
+    // the launches depend on the tiles only through the comparison with their blocks
+    const int nt = tables_.ntiles;
+    const bool divide = (nt < 2 * grid_.low) != (grid_.ntiles < 2 * grid_.low) ||
+                        (nt < 2 * grid_.pk) != (grid_.ntiles < 2 * grid_.pk);
+    if (variant != grid_.variant || mask != grid_.planes_mask || fermions != grid_.fermions || divide) {
         grid_ = eng_grid_size(low_, variant, full18_ ? 1 : 0, mask);
+        grid_.ntiles = nt;
         grid_.fermions = fermions;  // the phases the iteration launches (engine.cu)
         if (chunk_exec_) {
             HW_CUDA(cudaStreamSynchronize(ctx_->stream));

@@ -127,6 +127,29 @@ __device__ __forceinline__ void build_active(const EngPtrs &P, ActiveTable &A) {
     __syncthreads();
 }
 
+// Work items of the hop phases: a tile times a part of its active slots.  With fewer tiles
+// than twice the blocks, a tile's slots are divided (by a power of two) so that the launch has
+// about two items per block; every slot of a tile is still summed over the whole tile, so
+// results do not depend on the division.
+struct TileParts {
+    int shift = 0;  // 2^shift items per tile
+    __device__ TileParts() {}
+    __device__ explicit TileParts(int ntiles) {
+        while ((ntiles << shift) < 2 * (int)gridDim.x && (1 << shift) < kEngMaxRhs) shift++;
+    }
+    __device__ int items(int ntiles) const { return ntiles << shift; }
+    __device__ int tile(int item) const { return item >> shift; }
+    // slots [a0, a1) of na for the item's part, in multiples of `unit` (a power of two); false:
+    // nothing to do (the item still arrives: after the last arrival slots may leave, and the
+    // parts would shift)
+    __device__ bool range(int item, int na, int unit, int &a0, int &a1) const {
+        const int per = (((na + (1 << shift) - 1) >> shift) + unit - 1) & -unit;
+        a0 = (item & ((1 << shift) - 1)) * per;
+        a1 = min(na, a0 + per);
+        return a0 < na;
+    }
+};
+
 // ------------------------------------------------------------------ epilogues
 
 // Low-precision phases P1..P4.  acc = (H in)(i) in FP32.
@@ -378,7 +401,8 @@ __device__ __forceinline__ void arrive_and_finish(const EngPtrs &P, const EngLat
 // NR right-hand sides at a time, so links, their third rows and the neighbour
 // indices are shared by the NR solves.  PK (with NR = 2 and FP16 input): the two
 // solves run in the two lanes of packed FP32 instructions (pair.cuh).
-template <int PHASE, int LOW, int NR, int MINB, bool FULL18, bool PK = false>
+// PARTS: items divide a tile's slots (TileParts).
+template <int PHASE, int LOW, int NR, int MINB, bool FULL18, bool PK, bool PARTS>
 __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
     constexpr int SIGN = (PHASE == PH_P1 || PHASE == PH_P2) ? 1 : -1;
     constexpr int OUTPAR = (PHASE == PH_P1 || PHASE == PH_P3 || PHASE == PH_R4L) ? 1 : 0;
@@ -401,15 +425,18 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
     const int ntiles = T->ntiles;
     const int max_tiles = T->max_tiles;
     const bool dyn = T->dyn != 0;
-    // the next tile: block + k * grid, or the next value of the phase's counter; the
-    // partial sums are per (slot, tile), so the tile order does not change any result
-    auto next_tile = [&](int cur) {
+    const TileParts TP = PARTS ? TileParts(ntiles) : TileParts();
+    const int nitems = PARTS ? TP.items(ntiles) : ntiles;
+    // the next item: block + k * grid, or the next value of the phase's counter; the
+    // partial sums are per (slot, tile), so the order does not change any result
+    auto next_item = [&](int cur) {
         if (!dyn) return cur + (int)gridDim.x;
         if (threadIdx.x == 0) s_tile = atomicAdd(P.sched + PHASE, 1);
         __syncthreads();
         return s_tile;
     };
-    for (int tile = dyn ? next_tile(0) : (int)blockIdx.x; tile < ntiles; tile = next_tile(tile)) {
+    for (int item = dyn ? next_item(0) : (int)blockIdx.x; item < nitems; item = next_item(item)) {
+        const int tile = PARTS ? TP.tile(item) : item;
         const int l = find_lattice(T, tile);
         const EngLattice &La = T->lat[l];
         const Geom g = La.g;
@@ -432,7 +459,15 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
         }
         __syncthreads();
         const int na = s_na;
-        if (lt == 0 && threadIdx.x == 0 && na > 0) {
+        int a0 = 0, a1 = na;
+        if constexpr (PARTS) {
+            if (!TP.range(item, na, NR, a0, a1)) {
+                __syncthreads();  // s_act is rewritten by the next item
+                if constexpr (NRED > 0) arrive_and_finish<PHASE, NRED>(P, La, l, smem, last, TP.items(La.ntiles));
+                continue;
+            }
+        }
+        if (lt == 0 && threadIdx.x == 0 && na > 0 && a0 == 0) {
             count_work(P, PHASE, 0, (unsigned long long)na * g.Vh);
             count_work(P, PHASE, 2, g.Vh);
         }
@@ -445,8 +480,8 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
                 cp_async_wait_all();
             }
         }
-        for (int g0 = 0; g0 < na; g0 += NR) {
-            const int cnt = min(NR, na - g0);
+        for (int g0 = a0; g0 < a1; g0 += NR) {
+            const int cnt = min(NR, a1 - g0);
             // the reliable update of M x = b reads FP32 fields: s (in y) and t (in t64)
             constexpr bool ru32 = PHASE == PH_R4L || PHASE == PH_R5L;
             using InSp = typename std::conditional<ru32, SpinorF32, typename L::Sp>::type;
@@ -515,7 +550,7 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
         }
         if constexpr (NRED > 0) {
             __syncthreads();
-            if (threadIdx.x < na) {
+            if (threadIdx.x >= a0 && threadIdx.x < a1) {
                 double sum = 0;
 #pragma unroll
                 for (int w = 0; w < kEngTile / 32; w++) sum += s_red[threadIdx.x][w];
@@ -523,8 +558,8 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
                 __threadfence();  // visible before the lattice's ticket is taken
             }
         }
-        __syncthreads();  // s_act is rewritten by the next tile
-        if constexpr (NRED > 0) arrive_and_finish<PHASE, NRED>(P, La, l, smem, last, La.ntiles);
+        __syncthreads();  // s_act is rewritten by the next item
+        if constexpr (NRED > 0) arrive_and_finish<PHASE, NRED>(P, La, l, smem, last, PARTS ? TP.items(La.ntiles) : La.ntiles);
     }
 }
 
@@ -702,7 +737,7 @@ __global__ void k_eng_control(EngPtrs P, int nprob, int chunk, cudaGraphConditio
         if (s.status == ENG_RUNNING) atomicAdd(&running, 1);
     }
     __syncthreads();
-    if (threadIdx.x < kEngPhases) P.sched[threadIdx.x] = 0;  // the next iteration's tile counters
+    if (threadIdx.x < kEngPhases) P.sched[threadIdx.x] = 0;  // the next iteration's item counters
     if (threadIdx.x == 0) {
         if (chunk <= 0) chunk = P.ctl[3];
         const int it = P.ctl[0] + 1;
@@ -819,26 +854,39 @@ void enqueue_reliable_update(const EngPtrs &P, const EngGrid &G, cudaStream_t s,
     mark(ev, kEngPhases, s);
 }
 
-template <int LOW, int NR, int MINB, bool FULL18, bool PK = false>
+// One low-precision phase.  A launch with few tiles per block divides their slots (TileParts):
+// FP32, 3 sources at 20x12x28x36 (473 tiles for 888 blocks) P1 51 -> 45, P2 73 -> 64, P4 101 ->
+// 85 us; above two tiles per block the undivided form is as fast or faster (32^4).  (Blocks of
+// three teams on one tile, sharing its staged links and leaving more of the L1: P1 0.36 ->
+// 0.40 ms at 32^4 with 12 sources.)
+template <int PHASE, int LOW, int NR, int MINB, bool FULL18, bool PK = false>
+void launch_low(const EngPtrs &P, const EngGrid &G, int blocks, cudaStream_t s) {
+    if (G.ntiles < 2 * blocks)
+        k_eng_low<PHASE, LOW, NR, MINB, FULL18, PK, true><<<blocks, kEngTile, 0, s>>>(P);
+    else
+        k_eng_low<PHASE, LOW, NR, MINB, FULL18, PK, false><<<blocks, kEngTile, 0, s>>>(P);
+}
+
+template <int LOW, bool FULL18>
 struct LowShape {
     template <int PHASE>
     static void launch(const EngPtrs &P, const EngGrid &G, cudaStream_t s) {
-        k_eng_low<PHASE, LOW, NR, MINB, FULL18, PK><<<G.low, kEngTile, 0, s>>>(P);
+        launch_low<PHASE, LOW, 1, 6, FULL18>(P, G, G.low, s);
     }
 };
 
-template <int LOW, int NR, int MINB, bool FULL18, bool PK = false>
+template <int LOW, bool FULL18>
 void enqueue_iteration_t(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
     mark(ev, 0, s);
-    k_eng_low<PH_P1, LOW, NR, MINB, FULL18, PK><<<G.low, kEngTile, 0, s>>>(P);
+    launch_low<PH_P1, LOW, 1, 6, FULL18>(P, G, G.low, s);
     mark(ev, 1, s);
-    k_eng_low<PH_P2, LOW, NR, MINB, FULL18, PK><<<G.low, kEngTile, 0, s>>>(P);
+    launch_low<PH_P2, LOW, 1, 6, FULL18>(P, G, G.low, s);
     mark(ev, 2, s);
-    k_eng_low<PH_P3, LOW, NR, MINB, FULL18, PK><<<G.low, kEngTile, 0, s>>>(P);
+    launch_low<PH_P3, LOW, 1, 6, FULL18>(P, G, G.low, s);
     mark(ev, 3, s);
-    k_eng_low<PH_P4, LOW, NR, MINB, FULL18, PK><<<G.low, kEngTile, 0, s>>>(P);
+    launch_low<PH_P4, LOW, 1, 6, FULL18>(P, G, G.low, s);
     mark(ev, 4, s);
-    enqueue_reliable_update<LOW, LowShape<LOW, NR, MINB, FULL18, PK>>(P, G, s, ev);
+    enqueue_reliable_update<LOW, LowShape<LOW, FULL18>>(P, G, s, ev);
 }
 
 // P1 and P3 with two solves per thread in packed FP32 (MINB_PK blocks per SM, G.pk
@@ -846,15 +894,15 @@ void enqueue_iteration_t(const EngPtrs &P, const EngGrid &G, cudaStream_t s, con
 template <int LOW, int MINB_PK, bool FULL18>
 void enqueue_iteration_hybrid(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
     mark(ev, 0, s);
-    k_eng_low<PH_P1, LOW, 2, MINB_PK, FULL18, true><<<G.pk, kEngTile, 0, s>>>(P);
+    launch_low<PH_P1, LOW, 2, MINB_PK, FULL18, true>(P, G, G.pk, s);
     mark(ev, 1, s);
-    k_eng_low<PH_P2, LOW, 1, 6, FULL18><<<G.low, kEngTile, 0, s>>>(P);
+    launch_low<PH_P2, LOW, 1, 6, FULL18>(P, G, G.low, s);
     mark(ev, 2, s);
-    k_eng_low<PH_P3, LOW, 2, MINB_PK, FULL18, true><<<G.pk, kEngTile, 0, s>>>(P);
+    launch_low<PH_P3, LOW, 2, MINB_PK, FULL18, true>(P, G, G.pk, s);
     mark(ev, 3, s);
-    k_eng_low<PH_P4, LOW, 1, 6, FULL18><<<G.low, kEngTile, 0, s>>>(P);
+    launch_low<PH_P4, LOW, 1, 6, FULL18>(P, G, G.low, s);
     mark(ev, 4, s);
-    enqueue_reliable_update<LOW, LowShape<LOW, 1, 6, FULL18>>(P, G, s, ev);
+    enqueue_reliable_update<LOW, LowShape<LOW, FULL18>>(P, G, s, ev);
 }
 
 constexpr int kMmaMinBlocks = 4;
@@ -870,7 +918,7 @@ void enqueue_iteration_mma(const EngPtrs &P, const EngGrid &G, cudaStream_t s, c
     mark(ev, 3, s);
     k_eng_mma<PH_P4, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
     mark(ev, 4, s);
-    enqueue_reliable_update<LOW_F16, LowShape<LOW_F16, 1, 6, true>>(P, G, s, ev);
+    enqueue_reliable_update<LOW_F16, LowShape<LOW_F16, true>>(P, G, s, ev);
 }
 
 // Launch shapes of the low-precision phases (EngGrid::variant):
@@ -896,7 +944,7 @@ void enqueue_iteration_v(const EngPtrs &P, const EngGrid &G, cudaStream_t s, con
             return;
         }
     }
-    enqueue_iteration_t<LOW, 1, 6, FULL18>(P, G, s, ev);
+    enqueue_iteration_t<LOW, FULL18>(P, G, s, ev);
 }
 
 template <int LOW>
@@ -936,7 +984,7 @@ void eng_convert_links(const Geom &g, const double2 *l64, int planes, int stride
 template <int LOW, int NR, int MINB, bool PK = false, int PHASE = PH_P4>
 int occupancy_low() {
     int lo = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lo, k_eng_low<PHASE, LOW, NR, MINB, true, PK>, kEngTile, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lo, k_eng_low<PHASE, LOW, NR, MINB, true, PK, false>, kEngTile, 0);
     return lo < 1 ? 1 : lo;
 }
 
@@ -962,6 +1010,7 @@ EngGrid eng_grid_size(int low, int variant, int full18, int planes_mask) {
     if (variant == 7 && low == LOW_F16) G.pk = sms * occupancy_low<LOW_F16, 2, 3, true, PH_P1>();
     G.f64 = sms * (hi < 1 ? 1 : hi);
     G.fermions = 1;
+    G.ntiles = 0;
     G.variant = variant;
     G.full18 = full18;
     G.planes_mask = planes_mask;

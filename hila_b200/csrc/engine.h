@@ -150,6 +150,7 @@ struct EngGrid {
     int variant;  // launch shape of the low-precision phases (engine.cu)
     int full18;   // 1: inner phases read 18-real links (FP32 or FP16); 0: the 12-real links of the precision
     int planes_mask;  // FP64 link formats present: bit 0 = 18 reals, bit 1 = 12 reals
+    int ntiles;  // tiles the launches were shaped for (whether a tile's slots are divided)
     int fermions;     // lattice kinds present: bit 0 Wilson, bit 1 staggered (phases launched)
 };
 

@@ -70,7 +70,7 @@ int Engine::init() {
     if ((rc = d_tickets_.alloc(sizeof(unsigned) * kEngMaxLat)) != HW_OK) return rc;
     if ((rc = d_ctl_.alloc(sizeof(int) * 8)) != HW_OK) return rc;
     if ((rc = d_work_.alloc(sizeof(unsigned long long) * kEngPhases * kEngWorkKinds)) != HW_OK) return rc;
-    if ((rc = d_sched_.alloc(sizeof(int) * kEngPhases)) != HW_OK) return rc;
+    if ((rc = d_sched_.alloc(sizeof(int) * 2 * kEngPhases)) != HW_OK) return rc;
     HW_CUDA(cudaMemsetAsync(d_sched_.ptr, 0, d_sched_.bytes, ctx_->stream));
     HW_CUDA(cudaMemsetAsync(d_tickets_.ptr, 0, d_tickets_.bytes, ctx_->stream));
     HW_CUDA(cudaMemsetAsync(d_ctl_.ptr, 0, d_ctl_.bytes, ctx_->stream));
@@ -445,13 +445,19 @@ int Engine::build_graph() {
 }
 
 int Engine::configure() {
-    int mask = 0, fermions = 0;
-    for (int l = 0; l < tables_.nlat; l++) {
-        mask |= tables_.lat[l].l64_planes == 9 ? 1 : 2;
-        fermions |= 1 << tables_.lat[l].fermion;
-    }
+    int mask = 0, kinds = 0;
+    for (int l = 0; l < tables_.nlat; l++) mask |= tables_.lat[l].l64_planes == 9 ? 1 : 2;
+    for (int j = 0; j < kEngMaxProb; j++)
+        if (slots_[j].used) kinds |= 1 << host_states_[j].fermion;
     if (mask == 0) mask = 1;
-    if (fermions == 0) fermions = 1;
+    // a kind that was there keeps its phases for some chunks after its last slot has gone, so
+    // that a stream that alternates does not rebuild the graph each time
+    for (int k = 0; k < 3; k++) {
+        kind_idle_[k] = (kinds >> k & 1) ? 0 : kind_idle_[k] + 1;
+        if ((grid_.kinds >> k & 1) && kinds && kind_idle_[k] <= kKindIdleChunks && kind_seen_[k]) kinds |= 1 << k;
+        if (kinds >> k & 1) kind_seen_[k] = true;
+    }
+    if (kinds == 0) kinds = grid_.kinds;
     int variant = want_variant_ ? want_variant_ : default_variant();
     if (const char *env = std::getenv("HW_ENGINE_VARIANT")) variant = std::atoi(env);
     // launch shapes (engine.cu): 2 for both precisions, 4 and 7 for FP16 only; the
@@ -463,10 +469,10 @@ int Engine::configure() {
     const int nt = tables_.ntiles;
     const bool divide = (nt < 2 * grid_.low) != (grid_.ntiles < 2 * grid_.low) ||
                         (nt < 2 * grid_.pk) != (grid_.ntiles < 2 * grid_.pk);
-    if (variant != grid_.variant || mask != grid_.planes_mask || fermions != grid_.fermions || divide) {
+    if (variant != grid_.variant || mask != grid_.planes_mask || kinds != grid_.kinds || divide) {
         grid_ = eng_grid_size(low_, variant, full18_ ? 1 : 0, mask);
         grid_.ntiles = nt;
-        grid_.fermions = fermions;  // the phases the iteration launches (engine.cu)
+        grid_.kinds = kinds;  // the phases the iteration launches (engine.cu)
         if (chunk_exec_) {
             HW_CUDA(cudaStreamSynchronize(ctx_->stream));
             cudaGraphExecDestroy(chunk_exec_);

@@ -361,7 +361,7 @@ __device__ void finish(EngState &s, const EngProblem &pr, const double *tot, int
 // Arrival of one work item of lattice l (a tile, or a (tile, slot) pair: the
 // lattice expects `expected` of them); the last arrival sums every active
 // slot's partials in tile order and runs the finisher.
-template <int PHASE, int NRED, int FERM = FERM_WILSON>
+template <int PHASE, int NRED, int FERM = FERM_WILSON, int BLOCK = kEngTile>
 __device__ __forceinline__ void arrive_and_finish(const EngPtrs &P, const EngLattice &La, int l, double *smem,
                                                   bool &last, int expected) {
     const EngTables *T = P.T;
@@ -383,8 +383,8 @@ __device__ __forceinline__ void arrive_and_finish(const EngPtrs &P, const EngLat
             for (int k = 0; k < NRED; k++) {
                 const double *pp = P.partials + ((size_t)j * 2 + k) * max_tiles;
                 double s = 0.0;
-                for (int t2 = threadIdx.x; t2 < nt; t2 += kEngTile) s += __ldcg(pp + t2);
-                tot[k] = block_sum<kEngTile>(s, smem);
+                for (int t2 = threadIdx.x; t2 < nt; t2 += BLOCK) s += __ldcg(pp + t2);
+                tot[k] = block_sum<BLOCK>(s, smem);
             }
             if (threadIdx.x == 0) finish<PHASE>(P.S[j], T->prob[j], tot, P.ctl);
             __syncthreads();
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
         }
         SiteNbrs nb;
         if (valid && na > 0) nb = site_neighbours(g, i, OUTPAR);
-        const LinksF16x18Smem<kEngTile> US{s_lx, s_lz, OUTPAR};
+        const LinksF16x18Smem<kEngTile> US{s_lx, s_lz, OUTPAR, (int)threadIdx.x};
         if constexpr (STAGE) {
             if (valid && na > 0) {
                 US.stage(InnerLinks<LOW, FULL18>::lk(La), nb, i);
@@ -737,7 +737,7 @@ __global__ void k_eng_control(EngPtrs P, int nprob, int chunk, cudaGraphConditio
         if (s.status == ENG_RUNNING) atomicAdd(&running, 1);
     }
     __syncthreads();
-    if (threadIdx.x < kEngPhases) P.sched[threadIdx.x] = 0;  // the next iteration's item counters
+    if (threadIdx.x < 2 * kEngPhases) P.sched[threadIdx.x] = 0;  // the next iteration's item counters
     if (threadIdx.x == 0) {
         if (chunk <= 0) chunk = P.ctl[3];
         const int it = P.ctl[0] + 1;
@@ -751,7 +751,7 @@ __global__ void k_eng_control(EngPtrs P, int nprob, int chunk, cudaGraphConditio
 
 __global__ void k_eng_chunk_begin(EngPtrs P) {
     P.ctl[0] = 0;
-    for (int k = 0; k < kEngPhases; k++) P.sched[k] = 0;
+    for (int k = 0; k < 2 * kEngPhases; k++) P.sched[k] = 0;
 }
 
 // FP64 link planes (first six elements = rows 0 and 1) -> FP32 / FP16 12-real planes
@@ -958,14 +958,14 @@ void enqueue_iteration_nr(const EngPtrs &P, const EngGrid &G, cudaStream_t s, co
 }  // namespace
 
 void eng_enqueue_iteration(int low, const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
-    if (G.fermions & 1) {
+    if (G.kinds & 1) {
         if (low == LOW_F16)
             enqueue_iteration_nr<LOW_F16>(P, G, s, ev);
         else
             enqueue_iteration_nr<LOW_F32>(P, G, s, ev);
     }
     // staggered phases after the Wilson ones (outside the profiling events)
-    if (G.fermions & 2) enqueue_stag_iteration(P, G, s);
+    if (G.kinds & 6) enqueue_stag_iteration(P, G, s);
 }
 
 void eng_enqueue_control(const EngPtrs &P, int nprob, int chunk, cudaGraphConditionalHandle h, int use_cond,
@@ -1009,7 +1009,10 @@ EngGrid eng_grid_size(int low, int variant, int full18, int planes_mask) {
     G.pk = G.low;
     if (variant == 7 && low == LOW_F16) G.pk = sms * occupancy_low<LOW_F16, 2, 3, true, PH_P1>();
     G.f64 = sms * (hi < 1 ? 1 : hi);
-    G.fermions = 1;
+    int st = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&st, k_stag_low<PH_P4>, kStagLowBlock, 0);
+    G.stag = sms * (st < 1 ? 1 : st);
+    G.kinds = 1;
     G.ntiles = 0;
     G.variant = variant;
     G.full18 = full18;

@@ -129,8 +129,9 @@ struct EngPtrs {
                           // [2] reliable updates requested in this iteration,
                           // [3] iteration limit of a chunk (control kernel with chunk <= 0)
     unsigned long long *work;  // kEngPhases x kEngWorkKinds cumulative work units (below)
-    int *sched;           // kEngPhases tile counters of the inner phases' dynamic tile order
-                          // (zeroed at the start of a chunk and by every iteration's control kernel)
+    int *sched;           // item counters of the inner phases' dynamic order: kEngPhases of the Wilson
+                          // phases, then kEngPhases of the staggered FP16 ones (zeroed at the start
+                          // of a chunk and by every iteration's control kernel)
 };
 
 // Work units counted by every phase launch (cumulative, per phase), from which the
@@ -150,8 +151,9 @@ struct EngGrid {
     int variant;  // launch shape of the low-precision phases (engine.cu)
     int full18;   // 1: inner phases read 18-real links (FP32 or FP16); 0: the 12-real links of the precision
     int planes_mask;  // FP64 link formats present: bit 0 = 18 reals, bit 1 = 12 reals
+    int stag; // blocks of the staggered FP16 phases
     int ntiles;  // tiles the launches were shaped for (whether a tile's slots are divided)
-    int fermions;     // lattice kinds present: bit 0 Wilson, bit 1 staggered (phases launched)
+    int kinds;        // slot kinds whose phases are launched: bit 0 Wilson, bit 1 staggered FP64, bit 2 staggered FP16
 };
 
 // in launch order; R4 / R5 serve slots of the normal system (FP64), R4L / R5L those of

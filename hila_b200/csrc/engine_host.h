@@ -126,6 +126,9 @@ class Engine {
     int launch_chunk_profiled(int iters);
     int launch_chunk_timed(int iters);
     void tune_collect();
+    static constexpr int kKindIdleChunks = 16;
+    int kind_idle_[3] = {0, 0, 0};  // chunks since a slot of the kind was last in use (configure)
+    bool kind_seen_[3] = {false, false, false};
     int want_variant_ = 0;  // the tuner's shape for the next chunks (0: the default)
     std::map<int, TuneEntry> tune_;
     std::vector<cudaEvent_t> tune_ev_;  // kTuneMaxIters x (kEngPhases + 1)

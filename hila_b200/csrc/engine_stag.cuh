@@ -58,130 +58,174 @@ struct HalfStagY {
     }
 };
 
-// stag_hop_site in FP32 from FP16 fields and 18-real FP16 links (from memory, or the
-// tile's copy in shared memory); n: the neighbours of site i of output parity par
-template <class Lk>
-__device__ __forceinline__ void stag_hop_site_low(const Geom &g, const Lk &U, const SiteNbrs &n, int par, int i,
-                                                  const HalfStag16 &v, Cx<float> acc[3]) {
-    int c[4];
-    site_coords(g, i, par, c);
+// A thread of the FP16 phases serves two sources at a time, in the two lanes of packed FP32
+// instructions (pair.cuh); a block is two teams of kEngTile threads on the same sites, which
+// take the pairs of sources in turn and share the staged links.
+constexpr int kStagTeams = 2;
+constexpr int kStagLowBlock = kStagTeams * kEngTile;
+
+// the values of a pair of sources at one neighbour, as stored
+struct StagRaw {
+    uint4 a, b;
+    float na, nb;
+    __device__ __forceinline__ void load(const HalfStag16 &A, const HalfStag16 &B, int j) {
+        a = __ldg(A.p + j);
+        b = __ldg(B.p + j);
+        na = __ldg(A.n + j);
+        nb = __ldg(B.n + j);
+    }
+};
+
+// One term of the hop: acc += f U v (ADJ: f U^dag v), f the site norm of v times sg.  Lane
+// arithmetic is independent, so a source's result does not depend on the other; a source
+// without a partner fills both lanes.
+template <bool ADJ>
+__device__ __forceinline__ void stag_term(const Su3<float> &u, const StagRaw &raw, float sg, Cx2 (&acc)[3]) {
+    Cx2 w[3];
+    float2 nw[3];  // minus the part that the product subtracts
+    const __half2 *ha = reinterpret_cast<const __half2 *>(&raw.a);
+    const __half2 *hb = reinterpret_cast<const __half2 *>(&raw.b);
 #pragma unroll
-    for (int a = 0; a < 3; a++) acc[a] = {0.f, 0.f};
+    for (int c = 0; c < 3; c++) {
+        const float2 fa = __half22float2(ha[c]), fb = __half22float2(hb[c]);
+        w[c] = {make_float2(fa.x, fb.x), make_float2(fa.y, fb.y)};
+        nw[c] = neg2(ADJ ? w[c].re : w[c].im);
+    }
+    const float2 f = make_float2(sg * raw.na, sg * raw.nb);
 #pragma unroll
-    for (int d = 0; d < 4; d++) {
-        const float eta = (float)stag_eta(c, d);
-        const float sf = (d == 3 && n.tfwd_wrap) ? -eta : eta;
-        const float sb = (d == 3 && n.tbwd_wrap) ? -eta : eta;
-        Su3<float> u;
-        Cx<float> w[3];
-        U.load(par, d, i, u);
-        v.ld(n.fwd[d], w);
+    for (int a = 0; a < 3; a++) {
+        Cx2 t;
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const Cx<float> t = cmul(u.e[a][0], w[0]) + cmul(u.e[a][1], w[1]) + cmul(u.e[a][2], w[2]);
-            acc[a] = acc[a] + sf * t;
+        for (int c = 0; c < 3; c++) {
+            const Cx<float> e = ADJ ? u.e[c][a] : u.e[a][c];
+            const float2 er = bc2(e.re), ei = bc2(e.im);
+            t.re = c == 0 ? mul2(er, w[c].re) : fma2(er, w[c].re, t.re);
+            t.im = c == 0 ? mul2(er, w[c].im) : fma2(er, w[c].im, t.im);
+            t.re = fma2(ei, ADJ ? w[c].im : nw[c], t.re);
+            t.im = fma2(ei, ADJ ? nw[c] : w[c].re, t.im);
         }
-        U.load(1 - par, d, n.bwd[d], u);
-        v.ld(n.bwd[d], w);
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const Cx<float> t = cmul(conj(u.e[0][a]), w[0]) + cmul(conj(u.e[1][a]), w[1]) + cmul(conj(u.e[2][a]), w[2]);
-            acc[a] = acc[a] - sb * t;
-        }
+        acc[a] = axpy2(acc[a], f, t);
     }
 }
 
-// P1..P5 of a low-precision staggered slot at site i (FP32 arithmetic, FP16 fields);
-// red[0] receives the phase's |.|^2 contribution
-template <int PHASE, class Lk>
-__device__ __forceinline__ void stag_low_site(const EngLattice &La, const EngProblem &pr, const EngState &st,
-                                              const Lk &U, const SiteNbrs &nb, int i, double *red) {
-    constexpr int SIGN = (PHASE == PH_P1 || PHASE == PH_P2) ? 1 : -1;
-    constexpr int OUTPAR = (PHASE == PH_P1 || PHASE == PH_P3) ? 1 : 0;
-    const int stride = La.stride;
-    const float m = (float)pr.kappa;  // the mass
-    const HalfStag16 p{static_cast<uint4 *>(pr.p), pr.pn}, r{static_cast<uint4 *>(pr.r), pr.rn};
-    const HalfStag16 Dp{static_cast<uint4 *>(pr.Dp), pr.Dpn}, t{static_cast<uint4 *>(pr.t), pr.tn};
-    if constexpr (PHASE == PH_P5) {
-        Cx<float> rv[3], pv[3];
-        r.ld(i, rv);
-        if (!st.init) {
-            const float beta = (float)st.beta;
-            p.ldp(i, pv);
+// stag_hop_site in FP32 for a pair of sources; the next term's values are asked for before a
+// term is computed.  eta: bit d set for eta_d = +1.
+__device__ __forceinline__ void stag_hop_pair(const LinksF16x18Smem<kEngTile> &U, const SiteNbrs &n, unsigned eta,
+                                              int par, const HalfStag16 &A, const HalfStag16 &B, const StagRaw &first,
+                                              Cx2 (&acc)[3]) {
 #pragma unroll
-            for (int c = 0; c < 3; c++) rv[c] = rv[c] + beta * pv[c];
+    for (int a = 0; a < 3; a++) acc[a] = {bc2(0.f), bc2(0.f)};
+    StagRaw fw = first, bw;
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+        const float e = (eta >> d & 1u) ? 1.f : -1.f;
+        Su3<float> u;
+        bw.load(A, B, n.bwd[d]);
+        U.load(par, d, 0, u);
+        stag_term<false>(u, fw, (d == 3 && n.tfwd_wrap) ? -e : e, acc);
+        if (d < 3) fw.load(A, B, n.fwd[d + 1]);
+        U.load(1 - par, d, 0, u);
+        stag_term<true>(u, bw, (d == 3 && n.tbwd_wrap) ? e : -e, acc);
+    }
+}
+
+// the hop's input of a slot
+template <int PHASE>
+__device__ __forceinline__ HalfStag16 stag_low_in(const EngProblem &pr) {
+    if (PHASE == PH_P1) return HalfStag16{static_cast<uint4 *>(pr.p), pr.pn};
+    if (PHASE == PH_P3) return HalfStag16{static_cast<uint4 *>(pr.Dp), pr.Dpn};
+    return HalfStag16{static_cast<uint4 *>(pr.t), pr.tn};
+}
+
+// Own-site operands of a low-precision staggered slot's epilogue, and the epilogue: P1..P5 in
+// FP32 arithmetic on FP16 fields, acc the hop of the slot's input; red[0] receives the
+// phase's |.|^2 contribution.  The operands of two sources are loaded before either is used.
+template <int PHASE>
+struct StagOwn {
+    Cx<float> p[3], r[3], d[3], y[3];
+    __device__ __forceinline__ void load(const EngProblem &pr, int stride, int i) {
+        if constexpr (PHASE == PH_P2 || PHASE == PH_P4) HalfStag16{static_cast<uint4 *>(pr.p), pr.pn}.ld(i, p);
+        if constexpr (PHASE == PH_P4) {
+            HalfStag16{static_cast<uint4 *>(pr.Dp), pr.Dpn}.ld(i, d);
+            HalfStag16{static_cast<uint4 *>(pr.r), pr.rn}.ldp(i, r);
+            const HalfStagY Y{reinterpret_cast<float2 *>(pr.y), stride};
+#pragma unroll
+            for (int c = 0; c < 3; c++) y[c] = Y.ld(c, i);
         }
-        p.st(i, rv);
-    } else {
-        const HalfStag16 in = PHASE == PH_P1 ? p : PHASE == PH_P3 ? Dp : t;
-        Cx<float> acc[3], h[3];
-        stag_hop_site_low(La.g, U, nb, OUTPAR, i, in, acc);
+    }
+    __device__ __forceinline__ void finish(const EngProblem &pr, const EngState &st, int stride, int i,
+                                           const Cx<float> (&acc)[3], double *red) {
+        constexpr int SIGN = (PHASE == PH_P1 || PHASE == PH_P2) ? 1 : -1;
+        const float m = (float)pr.kappa;  // the mass
+        Cx<float> h[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) h[c] = (0.5f * SIGN) * acc[c];
-        if constexpr (OUTPAR == 1) {  // P1, P3: t = (1/m) D in
+        if constexpr (PHASE == PH_P1 || PHASE == PH_P3) {  // t = (1/m) D in
             const float im = 1.0f / m;
 #pragma unroll
             for (int c = 0; c < 3; c++) h[c] = im * h[c];
-            t.st(i, h);
+            HalfStag16{static_cast<uint4 *>(pr.t), pr.tn}.st(i, h);
         } else if constexpr (PHASE == PH_P2) {  // Dp = m p + D t
-            Cx<float> pv[3];
-            p.ld(i, pv);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                h[c] = m * pv[c] + h[c];
+                h[c] = m * p[c] + h[c];
                 red[0] += (double)norm2(h[c]);
             }
-            Dp.st(i, h);
+            HalfStag16{static_cast<uint4 *>(pr.Dp), pr.Dpn}.st(i, h);
         } else {  // P4: r -= alpha (m Dp + D t), y += alpha p
             const float alpha = (float)st.alpha;
-            Cx<float> dv[3], rv[3], pv[3];
-            Dp.ld(i, dv);
-            r.ldp(i, rv);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                rv[c] = rv[c] - alpha * (m * dv[c] + h[c]);
-                red[0] += (double)norm2(rv[c]);
+                r[c] = r[c] - alpha * (m * d[c] + h[c]);
+                red[0] += (double)norm2(r[c]);
             }
-            r.st(i, rv);
-            p.ld(i, pv);
-            const HalfStagY y{reinterpret_cast<float2 *>(pr.y), stride};
+            HalfStag16{static_cast<uint4 *>(pr.r), pr.rn}.st(i, r);
+            const HalfStagY Y{reinterpret_cast<float2 *>(pr.y), stride};
 #pragma unroll
-            for (int c = 0; c < 3; c++) y.st(c, i, y.ld(c, i) + alpha * pv[c]);
+            for (int c = 0; c < 3; c++) Y.st(c, i, y[c] + alpha * p[c]);
         }
     }
-}
+};
 
-// P1..P5 of the staggered slots with FP16 inner iterations, in the shape of the Wilson
-// inner phases: a block walks tiles (block + k x grid); per tile, the sites' eight FP16
-// links are copied into shared memory once and read from there by every such slot of the
-// lattice, and each slot's partial sum is formed once per tile in block_sum's order.
+// P1..P4 of the staggered slots with FP16 inner iterations: a block takes items (a tile and a
+// part of its slots) from a counter; per item, the sites' eight FP16 links are copied into
+// shared memory once, the block's teams take the pairs of slots in turn, and each slot's partial
+// sum is formed once per tile in block_sum's order.
 template <int PHASE>
-__global__ void __launch_bounds__(kEngTile, 4) k_stag_low(EngPtrs P) {
+__global__ void __launch_bounds__(kStagLowBlock, 3) k_stag_low(EngPtrs P) {
     constexpr int OUTPAR = (PHASE == PH_P1 || PHASE == PH_P3) ? 1 : 0;
     constexpr int NRED = (PHASE == PH_P2 || PHASE == PH_P4) ? 1 : 0;
-    constexpr bool HOP = PHASE != PH_P5;
-    __shared__ double smem[kEngTile / 32];
+    __shared__ double smem[kStagLowBlock / 32];
     __shared__ bool last;
+    __shared__ int s_item;
     __shared__ int s_act[kEngMaxRhs];
     __shared__ int s_na;
-    __shared__ uint4 s_lx[HOP ? 16 * kEngTile : 1];
-    __shared__ unsigned s_lz[HOP ? 8 * kEngTile : 1];
+    __shared__ uint4 s_lx[16 * kEngTile];
+    __shared__ unsigned s_lz[8 * kEngTile];
     __shared__ double s_red[NRED > 0 ? kEngMaxRhs : 1][kEngTile / 32];
     const EngTables *T = P.T;
-    const int ntiles = T->ntiles;
     const int max_tiles = T->max_tiles;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const TileParts TP(T->ntiles);
+    const int nitems = TP.items(T->ntiles);
+    const int team = threadIdx.x / kEngTile, t = threadIdx.x % kEngTile;
+    const LinksF16x18Smem<kEngTile> US{s_lx, s_lz, OUTPAR, t};
+    auto next_item = [&]() {
+        if (threadIdx.x == 0) s_item = atomicAdd(P.sched + kEngPhases + PHASE, 1);
+        __syncthreads();
+        return s_item;
+    };
+    for (int item = next_item(); item < nitems; item = next_item()) {
+        const int tile = TP.tile(item);
         const int l = find_lattice(T, tile);
         const EngLattice &La = T->lat[l];
-        if (La.fermion != FERM_STAGGERED) continue;
         const int lt = tile - La.tile0;
-        const int i = lt * kEngTile + threadIdx.x;
+        const int i = lt * kEngTile + t;
         const bool valid = i < La.g.Vh;
         if (threadIdx.x < 32) {
             const int q = threadIdx.x;
             int j = 0;
             bool on = false;
-            if (q < La.nprob) {
+            if (La.fermion == FERM_STAGGERED && q < La.nprob) {
                 j = La.prob[q];
                 on = active<PHASE, FERM_STAGGERED_LOW>(P.S[j]);
             }
@@ -191,33 +235,71 @@ __global__ void __launch_bounds__(kEngTile, 4) k_stag_low(EngPtrs P) {
         }
         __syncthreads();
         const int na = s_na;
-        // every tile of a lattice sees the same active slots: a lattice without any is left
+        // every item of a lattice sees the same active slots: a lattice without any is left
         // alone (no arrival, its ticket untouched)
-        if (na == 0) {
+        int a0, a1;
+        if (!TP.range(item, na, 2, a0, a1)) {
             __syncthreads();
+            if (NRED > 0 && na > 0)
+                arrive_and_finish<PHASE, NRED, FERM_STAGGERED_LOW, kStagLowBlock>(P, La, l, smem, last,
+                                                                                 TP.items(La.ntiles));
             continue;
         }
-        const LinksF16x18Smem<kEngTile> US{s_lx, s_lz, OUTPAR};
         SiteNbrs nb;
-        if constexpr (HOP) {
-            if (valid) {
-                nb = site_neighbours(La.g, i, OUTPAR);
-                US.stage(LinksF16x18{La.l16x, La.l16z, La.stride}, nb, i);
-                cp_async_wait_all();
-            }
+        unsigned eta = 0;
+        if (valid) {
+            nb = site_neighbours(La.g, i, OUTPAR);
+            US.stage<kStagTeams>(LinksF16x18{La.l16x, La.l16z, La.stride}, nb, i, team);
+            int c[4];
+            site_coords(La.g, i, OUTPAR, c);
+#pragma unroll
+            for (int d = 0; d < 4; d++) eta |= (stag_eta(c, d) > 0.0 ? 1u : 0u) << d;
         }
-        for (int a = 0; a < na; a++) {
-            const int j = s_act[a];
-            double red[1] = {0.0};
-            if (valid) stag_low_site<PHASE>(La, T->prob[j], P.S[j], US, nb, i, red);
+        const int stride = La.stride;
+        bool staged = false;
+        for (int a = a0; a < a1; a += 2 * kStagTeams) {
+            const int mine = a + 2 * team;  // this team's pair of slots
+            const bool on = valid && mine < a1;
+            const bool two = mine + 1 < a1;
+            const int jA = s_act[min(mine, a1 - 1)], jB = s_act[min(mine + 1, a1 - 1)];
+            const EngProblem &A = T->prob[jA], &B = T->prob[jB];
+            const HalfStag16 inA = stag_low_in<PHASE>(A), inB = stag_low_in<PHASE>(B);
+            StagRaw first;
+            if (on) first.load(inA, inB, nb.fwd[0]);
+            if (!staged) {  // each team copied half of the links
+                cp_async_wait_all();
+                __syncthreads();
+                staged = true;
+            }
+            double redA = 0.0, redB = 0.0;
+            if (on) {
+                Cx2 acc[3];
+                stag_hop_pair(US, nb, eta, OUTPAR, inA, inB, first, acc);
+                StagOwn<PHASE> oa, ob;
+                oa.load(A, stride, i);
+                if (two) ob.load(B, stride, i);
+                Cx<float> ha[3], hb[3];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    ha[c] = {acc[c].re.x, acc[c].im.x};
+                    hb[c] = {acc[c].re.y, acc[c].im.y};
+                }
+                oa.finish(A, P.S[jA], stride, i, ha, &redA);
+                if (two) ob.finish(B, P.S[jB], stride, i, hb, &redB);
+            }
             if constexpr (NRED > 0) {
-                const double v = warp_sum(red[0]);
-                if ((threadIdx.x & 31) == 0) s_red[a][threadIdx.x >> 5] = v;
+                if (mine < a1) {
+                    const double vA = warp_sum(redA), vB = warp_sum(redB);
+                    if ((t & 31) == 0) {
+                        s_red[mine][t >> 5] = vA;
+                        if (two) s_red[mine + 1][t >> 5] = vB;
+                    }
+                }
             }
         }
         if constexpr (NRED > 0) {
             __syncthreads();
-            if (threadIdx.x < na) {
+            if (threadIdx.x >= a0 && threadIdx.x < a1) {
                 double sum = 0;
 #pragma unroll
                 for (int w = 0; w < kEngTile / 32; w++) sum += s_red[threadIdx.x][w];
@@ -225,8 +307,49 @@ __global__ void __launch_bounds__(kEngTile, 4) k_stag_low(EngPtrs P) {
                 __threadfence();  // visible before the lattice's ticket is taken
             }
         }
-        __syncthreads();  // s_act and the staged links are rewritten by the next tile
-        if constexpr (NRED > 0) arrive_and_finish<PHASE, NRED, FERM_STAGGERED_LOW>(P, La, l, smem, last, La.ntiles);
+        __syncthreads();  // s_act and the staged links are rewritten by the next item
+        if constexpr (NRED > 0)
+            arrive_and_finish<PHASE, NRED, FERM_STAGGERED_LOW, kStagLowBlock>(P, La, l, smem, last,
+                                                                             TP.items(La.ntiles));
+    }
+}
+
+// P5 of those slots: p = r + beta p (p = r in a slot's first iteration), the slots of a tile
+// four at a time so that their loads are in flight together
+constexpr int kStagP5Src = 4;
+__global__ void __launch_bounds__(kEngTile) k_stag_low_p5(EngPtrs P) {
+    const EngTables *T = P.T;
+    for (int tile = blockIdx.x; tile < T->ntiles; tile += gridDim.x) {
+        const int l = find_lattice(T, tile);
+        const EngLattice &La = T->lat[l];
+        if (La.fermion != FERM_STAGGERED) continue;
+        const int i = (tile - La.tile0) * kEngTile + threadIdx.x;
+        if (i >= La.g.Vh) continue;
+        for (int q0 = 0; q0 < La.nprob; q0 += kStagP5Src) {
+            Cx<float> r[kStagP5Src][3], p[kStagP5Src][3];
+            bool on[kStagP5Src];
+#pragma unroll
+            for (int k = 0; k < kStagP5Src; k++) {
+                on[k] = q0 + k < La.nprob && active<PH_P5, FERM_STAGGERED_LOW>(P.S[La.prob[q0 + k]]);
+                if (on[k]) {
+                    const EngProblem &pr = T->prob[La.prob[q0 + k]];
+                    HalfStag16{static_cast<uint4 *>(pr.r), pr.rn}.ld(i, r[k]);
+                    HalfStag16{static_cast<uint4 *>(pr.p), pr.pn}.ldp(i, p[k]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kStagP5Src; k++)
+                if (on[k]) {
+                    const int j = La.prob[q0 + k];
+                    const EngProblem &pr = T->prob[j];
+                    const EngState &st = P.S[j];
+                    const float beta = (float)st.beta;
+                    if (!st.init)
+#pragma unroll
+                        for (int c = 0; c < 3; c++) r[k][c] = r[k][c] + beta * p[k][c];
+                    HalfStag16{static_cast<uint4 *>(pr.p), pr.pn}.st(i, r[k]);
+                }
+        }
     }
 }
 
@@ -396,18 +519,19 @@ __global__ void __launch_bounds__(kEngTile, 3) k_stag_eng(EngPtrs P) {
     }
 }
 
-// one iteration of the staggered slots (the reliable-update phases return at once unless
-// some slot asked for one)
+// one iteration of the staggered slots: the phases of the slot kinds present (FP64 and FP16
+// slots of a phase are disjoint; each kernel finishes its own); the reliable-update phases,
+// which serve both kinds, return at once unless some slot asked for one
 void enqueue_stag_iteration(const EngPtrs &P, const EngGrid &G, cudaStream_t s) {
-    // FP64 and FP16 slots of a phase are disjoint; each kernel finishes its own
-    k_stag_eng<PH_P1><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_low<PH_P1><<<G.low, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_P2><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_low<PH_P2><<<G.low, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_P3><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_low<PH_P3><<<G.low, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_P4><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_low<PH_P4><<<G.low, kEngTile, 0, s>>>(P);
+    const bool f64 = G.kinds & 2, low = G.kinds & 4;
+    if (f64) k_stag_eng<PH_P1><<<G.f64, kEngTile, 0, s>>>(P);
+    if (low) k_stag_low<PH_P1><<<G.stag, kStagLowBlock, 0, s>>>(P);
+    if (f64) k_stag_eng<PH_P2><<<G.f64, kEngTile, 0, s>>>(P);
+    if (low) k_stag_low<PH_P2><<<G.stag, kStagLowBlock, 0, s>>>(P);
+    if (f64) k_stag_eng<PH_P3><<<G.f64, kEngTile, 0, s>>>(P);
+    if (low) k_stag_low<PH_P3><<<G.stag, kStagLowBlock, 0, s>>>(P);
+    if (f64) k_stag_eng<PH_P4><<<G.f64, kEngTile, 0, s>>>(P);
+    if (low) k_stag_low<PH_P4><<<G.stag, kStagLowBlock, 0, s>>>(P);
     k_stag_eng<PH_R1><<<G.f64, kEngTile, 0, s>>>(P);
     k_stag_eng<PH_R2><<<G.f64, kEngTile, 0, s>>>(P);
     k_stag_eng<PH_R3><<<G.f64, kEngTile, 0, s>>>(P);
@@ -415,6 +539,6 @@ void enqueue_stag_iteration(const EngPtrs &P, const EngGrid &G, cudaStream_t s) 
     k_stag_eng<PH_R4L><<<G.f64, kEngTile, 0, s>>>(P);
     k_stag_eng<PH_R5><<<G.f64, kEngTile, 0, s>>>(P);
     k_stag_eng<PH_R5L><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_P5><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_low<PH_P5><<<G.low, kEngTile, 0, s>>>(P);
+    if (f64) k_stag_eng<PH_P5><<<G.f64, kEngTile, 0, s>>>(P);
+    if (low) k_stag_low_p5<<<4 * G.stag, kEngTile, 0, s>>>(P);
 }

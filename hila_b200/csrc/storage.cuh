@@ -353,17 +353,20 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // The eight links of the hop at one output site (forward U_mu(x) in slots 0..3,
 // backward U_mu(x - mu) in slots 4..7) of 18-real FP16 links, copied once into
 // shared memory and read from there by every right-hand side of the site.
-// Slot k of thread t: x[(2k + w) * BLOCK + t] (w = 0, 1), z[k * BLOCK + t].
+// Slot k of site t: x[(2k + w) * BLOCK + t] (w = 0, 1), z[k * BLOCK + t].
 template <int BLOCK>
 struct LinksF16x18Smem {
     using R = float;
     uint4 *x;
     unsigned *z;
     int outpar;  // parity of the output site: par == outpar selects the forward slots
-    __device__ __forceinline__ void stage(const LinksF16x18 &U, const SiteNbrs &n, int i) const {
-        const int t = threadIdx.x;
+    int t;       // site of the tile
+    // TEAMS teams of BLOCK threads copy the slots in turn; the block meets before they are read
+    template <int TEAMS = 1>
+    __device__ __forceinline__ void stage(const LinksF16x18 &U, const SiteNbrs &n, int i, int team = 0) const {
 #pragma unroll
         for (int k = 0; k < 8; k++) {
+            if (TEAMS > 1 && k % TEAMS != team) continue;
             const int dir = k & 3;
             const int pd = (k < 4 ? outpar : 1 - outpar) * 4 + dir;
             const int idx = k < 4 ? i : n.bwd[dir];
@@ -374,7 +377,6 @@ struct LinksF16x18Smem {
     }
     __device__ __forceinline__ void load(int par, int dir, int, Su3<float> &u) const {
         const int k = (par == outpar ? 0 : 4) + dir;
-        const int t = threadIdx.x;
         const uint4 a[2] = {x[(2 * k) * BLOCK + t], x[(2 * k + 1) * BLOCK + t]};
         LinksF16x18::unpack(a, z[k * BLOCK + t], u);
     }

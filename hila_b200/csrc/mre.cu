@@ -14,6 +14,7 @@
 // direction whose pivot is below 1e-16 (MRE_guess.h:55-80).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -26,18 +27,34 @@ namespace {
 constexpr int kMreBlock = 256;
 constexpr int kMreMaxBlocks = 1024;
 
-// per-block partial of Re sum_i conj(a_i) b_i over EVEN sites (fixed grid-stride and tree order)
-__global__ void __launch_bounds__(kMreBlock) k_rdot(int Vh, HalfF64 a, HalfF64 b, double *partials) {
-    __shared__ double smem[kMreBlock / 32];
-    double s = 0.0;
+// out[0] = Re sum_i conj(a_i) b_i over EVEN sites (fixed grid-stride, tree and block order)
+struct StoreSum {
+    double *out;
+    __device__ void operator()(const double *tot) const { *out = tot[0]; }
+};
+__global__ void __launch_bounds__(kMreBlock) k_rdot(int Vh, HalfF64 a, HalfF64 b, StoreSum fin, RedBuf red) {
+    double s[1] = {0.0};
     for (int i = blockIdx.x * kMreBlock + threadIdx.x; i < Vh; i += gridDim.x * kMreBlock)
 #pragma unroll
         for (int c = 0; c < 12; c++) {
             const double2 u = a.p[(size_t)c * a.stride + i], v = b.p[(size_t)c * b.stride + i];
-            s += u.x * v.x + u.y * v.y;
+            s[0] += u.x * v.x + u.y * v.y;
         }
-    const double t = block_sum<kMreBlock>(s, smem);
-    if (threadIdx.x == 0) partials[blockIdx.x] = t;
+    grid_reduce<1, kMreBlock>(s, red.partials, red.ticket, fin);
+}
+
+// y -= (ov / n2) x over EVEN sites with the scalars on the device; left alone for a null x
+__global__ void __launch_bounds__(kMreBlock) k_project_out(int Vh, const double *ov, const double *n2, HalfF64 x,
+                                                          HalfF64 y) {
+    if (!(*n2 > 1e-300)) return;
+    const double a = -*ov / *n2;
+    for (int i = blockIdx.x * kMreBlock + threadIdx.x; i < Vh; i += gridDim.x * kMreBlock)
+#pragma unroll
+        for (int c = 0; c < 12; c++) {
+            const double2 u = x.p[(size_t)c * x.stride + i];
+            double2 &v = y.p[(size_t)c * y.stride + i];
+            v = make_double2(v.x + a * u.x, v.y + a * u.y);
+        }
 }
 
 // y += a x over EVEN sites
@@ -51,29 +68,20 @@ __global__ void __launch_bounds__(kMreBlock) k_axpy(int Vh, double a, HalfF64 x,
         }
 }
 
+// The scalars stay on the device until the projected system is complete: one read back instead
+// of one for each of the n (3 n + 3) / 2 products.
 struct Mre {
     hw_context *ctx;
     int Vh;
     int blocks;
-    DevBuf partials;
-    std::vector<double> host;
 
-    int rdot(HalfF64 a, HalfF64 b, double *out) {
-        k_rdot<<<blocks, kMreBlock, 0, ctx->stream>>>(Vh, a, b, partials.as<double>());
-        HW_CUDA(cudaGetLastError());
-        HW_CUDA(cudaMemcpyAsync(host.data(), partials.ptr, sizeof(double) * blocks, cudaMemcpyDeviceToHost,
-                                ctx->stream));
-        HW_CUDA(cudaStreamSynchronize(ctx->stream));
-        double s = 0.0;
-        for (int k = 0; k < blocks; k++) s += host[k];
-        *out = s;
-        return HW_OK;
+    void rdot(HalfF64 a, HalfF64 b, double *out) {
+        k_rdot<<<blocks, kMreBlock, 0, ctx->stream>>>(Vh, a, b, StoreSum{out}, ctx->red());
     }
-    int axpy(double a, HalfF64 x, HalfF64 y) {
-        k_axpy<<<blocks, kMreBlock, 0, ctx->stream>>>(Vh, a, x, y);
-        HW_CUDA(cudaGetLastError());
-        return HW_OK;
+    void project_out(const double *ov, const double *n2, HalfF64 x, HalfF64 y) {
+        k_project_out<<<blocks, kMreBlock, 0, ctx->stream>>>(Vh, ov, n2, x, y);
     }
+    void axpy(double a, HalfF64 x, HalfF64 y) { k_axpy<<<blocks, kMreBlock, 0, ctx->stream>>>(Vh, a, x, y); }
 };
 
 }  // namespace
@@ -101,36 +109,36 @@ extern "C" int hw_mre_guess(const hw_gauge *gauge, double kappa, double mh, cons
     m.ctx = ctx;
     m.Vh = (int)lat->Vh;
     m.blocks = (int)std::min<long>((lat->Vh + kMreBlock - 1) / kMreBlock, kMreMaxBlocks);
-    m.host.resize(m.blocks);
-    if ((rc = m.partials.alloc(sizeof(double) * m.blocks)) != HW_OK) return rc;
-    std::vector<DevBuf> basis(n);
-    DevBuf t1, t2;
-    if ((rc = t1.alloc(half_bytes)) != HW_OK) return rc;
-    if ((rc = t2.alloc(half_bytes)) != HW_OK) return rc;
-    auto h = [stride](const DevBuf &b) { return HalfF64{b.as<double2>(), stride}; };
+    // the basis in one block of memory; device scalars: overlap, |b_i|^2, M, v
+    DevBuf basis, scal;
+    if ((rc = basis.alloc(n * half_bytes)) != HW_OK) return rc;
+    if ((rc = scal.alloc((1 + 2 * n + (size_t)n * n) * sizeof(double))) != HW_OK) return rc;
+    double *ov = scal.as<double>(), *bb = ov + 1, *dM = bb + n, *dv = dM + (size_t)n * n;
+    auto h = [&](int i) { return HalfF64{basis.as<double2>() + (size_t)i * 12 * stride, stride}; };
+    const HalfF64 t1 = lat->ws->Dp.h(), t2 = lat->ws->DDp.h();
     // orthogonalised basis: b_i = old_i - sum_{j<i} (Re<b_j, b_i> / |b_j|^2) b_j
-    std::vector<double> bb(n, 0.0);
     for (int i = 0; i < n; i++) {
-        if ((rc = basis[i].alloc(half_bytes)) != HW_OK) return rc;
-        HW_CUDA(cudaMemcpyAsync(basis[i].ptr, old[i]->half[0].buf.ptr, half_bytes, cudaMemcpyDeviceToDevice,
-                                ctx->stream));
+        HW_CUDA(cudaMemcpyAsync(h(i).p, old[i]->half[0].buf.ptr, half_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
         for (int j = 0; j < i; j++) {
-            if (!(bb[j] > 1e-300)) continue;
-            double ov;
-            if ((rc = m.rdot(h(basis[j]), h(basis[i]), &ov)) != HW_OK) return rc;
-            if ((rc = m.axpy(-ov / bb[j], h(basis[j]), h(basis[i]))) != HW_OK) return rc;
+            m.rdot(h(j), h(i), ov);
+            m.project_out(ov, bb + j, h(j), h(i));
         }
-        if ((rc = m.rdot(h(basis[i]), h(basis[i]), &bb[i])) != HW_OK) return rc;
+        m.rdot(h(i), h(i), bb + i);
     }
     // projected system  M[j][i] = Re<b_j, A b_i>,  v[i] = Re<b_i, chi>
     const double d = 1.0 + mh;
-    std::vector<double> Mm((size_t)n * n), v(n);
     for (int i = 0; i < n; i++) {
-        eo_apply_half(gauge, kappa, h(basis[i]), h(t1), +1, d);
-        eo_apply_half(gauge, kappa, h(t1), h(t2), -1, d);
-        for (int j = 0; j < n; j++)
-            if ((rc = m.rdot(h(basis[j]), h(t2), &Mm[(size_t)j * n + i])) != HW_OK) return rc;
-        if ((rc = m.rdot(h(basis[i]), chi->half[0].h(), &v[i])) != HW_OK) return rc;
+        eo_apply_half(gauge, kappa, h(i), t1, +1, d);
+        eo_apply_half(gauge, kappa, t1, t2, -1, d);
+        for (int j = 0; j < n; j++) m.rdot(h(j), t2, dM + (size_t)j * n + i);
+        m.rdot(h(i), chi->half[0].h(), dv + i);
+    }
+    HW_CUDA(cudaGetLastError());
+    std::vector<double> Mm((size_t)n * n), v(n);
+    if (n) {
+        HW_CUDA(cudaMemcpyAsync(Mm.data(), dM, Mm.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        HW_CUDA(cudaMemcpyAsync(v.data(), dv, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        HW_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     // Gauss-Jordan elimination (MRE_guess.h:55-80)
     for (int i = 0; i < n; i++) {
@@ -155,8 +163,8 @@ extern "C" int hw_mre_guess(const hw_gauge *gauge, double kappa, double mh, cons
     HW_CUDA(cudaMemsetAsync(psi->half[0].buf.ptr, 0, psi->half[0].buf.bytes, ctx->stream));
     HW_CUDA(cudaMemsetAsync(psi->half[1].buf.ptr, 0, psi->half[1].buf.bytes, ctx->stream));
     for (int i = 0; i < n; i++)
-        if (std::isfinite(v[i]) && v[i] != 0.0)
-            if ((rc = m.axpy(v[i], h(basis[i]), psi->half[0].h())) != HW_OK) return rc;
+        if (std::isfinite(v[i]) && v[i] != 0.0) m.axpy(v[i], h(i), psi->half[0].h());
+    HW_CUDA(cudaGetLastError());
     HW_CUDA(cudaStreamSynchronize(ctx->stream));
     return HW_OK;
 }

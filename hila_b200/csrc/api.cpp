@@ -178,6 +178,7 @@ int hw_context_destroy(hw_context *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     destroy_engines(ctx);
+    ctx->copier.reset();
     if (ctx->cg_state_host) cudaFreeHost(ctx->cg_state_host);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -336,9 +337,7 @@ int hw_field_download(const hw_field *f, double *host, int parity) {
     for (int p = 0; p < 2; p++)
         if (parity & (1 << p)) launch_spinor_eo_to_lex(lat->g, f->half[p].h(), p, stage.as<double>(), ctx->stream);
     HW_CUDA(cudaGetLastError());
-    HW_CUDA(cudaMemcpyAsync(host, stage.ptr, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    HW_CUDA(cudaStreamSynchronize(ctx->stream));
-    return HW_OK;
+    return copy_to_host(ctx, host, stage.ptr, bytes);
 }
 
 int hw_field_upload_eo(hw_field *f, const double *host, int parity) {
@@ -375,11 +374,9 @@ int hw_field_download_eo(const hw_field *f, double *host, int parity) {
     for (int p = 0; p < 2; p++)
         if (parity & (1 << p)) {
             launch_soa_to_aos((int)lat->Vh, f->half[p].h(), ctx->stage.as<double>(), ctx->stream);
-            HW_CUDA(cudaMemcpyAsync(host + p * half, ctx->stage.ptr, half * sizeof(double), cudaMemcpyDeviceToHost,
-                                    ctx->stream));
+            HW_CUDA(cudaGetLastError());
+            if ((rc = copy_to_host(ctx, host + p * half, ctx->stage.ptr, half * sizeof(double))) != HW_OK) return rc;
         }
-    HW_CUDA(cudaGetLastError());
-    HW_CUDA(cudaStreamSynchronize(ctx->stream));
     return HW_OK;
 }
 

@@ -116,13 +116,14 @@ extern "C" int hw_wilson_evenodd_force(const hw_gauge *gauge, double kappa, cons
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     HW_CUDA(cudaSetDevice(ctx->device));
     int rc;
+    if ((rc = ensure_workspace(lat)) != HW_OK) return rc;
     if ((rc = tune_hop(lat, gauge)) != HW_OK) return rc;
     const int stride = lat->stride;
-    DevBuf t1, t2, out;
-    if ((rc = t1.alloc((size_t)12 * stride * sizeof(double2))) != HW_OK) return rc;
-    if ((rc = t2.alloc((size_t)12 * stride * sizeof(double2))) != HW_OK) return rc;
-    if ((rc = out.alloc((size_t)36 * lat->V * sizeof(double2))) != HW_OK) return rc;
-    const HalfF64 h1{t1.as<double2>(), stride}, h2{t2.as<double2>(), stride};
+    DevBuf own;
+    void *out = nullptr;
+    const size_t bytes = (size_t)36 * lat->V * sizeof(double2);
+    if ((rc = force_buffer(ctx, bytes, own, &out)) != HW_OK) return rc;
+    const HalfF64 h1 = lat->ws->t.h(), h2 = lat->ws->res.h();
     // t1 = -kappa H^{oe}_{-s} chi, t2 = -kappa H^{oe}_s psi (wilson.h:298-307)
     launch_hop_scale(lat->g, gauge->U(), 1, -sign, chi->half[0].h(), h1, -kappa, nullptr, ctx->stream);
     launch_hop_scale(lat->g, gauge->U(), 1, sign, psi->half[0].h(), h2, -kappa, nullptr, ctx->stream);
@@ -134,11 +135,9 @@ extern "C" int hw_wilson_evenodd_force(const hw_gauge *gauge, double kappa, cons
     const SpinorF64 c{chi->half[0].buf.as<double2>(), stride}, p{psi->half[0].buf.as<double2>(), stride};
     const SpinorF64 s1{h1.p, stride}, s2{h2.p, stride};
     if (sign > 0)
-        k_eo_force<1><<<grid, kForceBlock, 0, ctx->stream>>>(lat->g, c, p, s1, s2, kappa, lat->V, out.as<double2>());
+        k_eo_force<1><<<grid, kForceBlock, 0, ctx->stream>>>(lat->g, c, p, s1, s2, kappa, lat->V, static_cast<double2 *>(out));
     else
-        k_eo_force<-1><<<grid, kForceBlock, 0, ctx->stream>>>(lat->g, c, p, s1, s2, kappa, lat->V, out.as<double2>());
+        k_eo_force<-1><<<grid, kForceBlock, 0, ctx->stream>>>(lat->g, c, p, s1, s2, kappa, lat->V, static_cast<double2 *>(out));
     HW_CUDA(cudaGetLastError());
-    HW_CUDA(cudaMemcpyAsync(force, out.ptr, out.bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    HW_CUDA(cudaStreamSynchronize(ctx->stream));
-    return HW_OK;
+    return copy_to_host(ctx, force, out, bytes);
 }

@@ -55,6 +55,16 @@ struct DevBuf {
     }
 };
 
+// Threads, page-locked chunks and streams of the copies into pageable memory (host_copy.cpp),
+// kept by the context (8 MiB)
+constexpr int kCopyWorkers = 8;
+struct HostCopier {
+    void *buf[kCopyWorkers] = {};
+    cudaStream_t stream[kCopyWorkers] = {};
+    int init();
+    ~HostCopier();
+};
+
 // Sites per parity rounded up to 64 so every SoA plane starts 1 KiB aligned
 // (for FP64 planes) and coalesced rows never straddle planes.
 inline int padded_stride(long vh) { return (int)((vh + 63) / 64 * 64); }
@@ -73,6 +83,7 @@ struct hw_context {
     hw::DevBuf stage;         // lexicographic staging buffer for host transfers (grow-only)
     hw::CgState *cg_state_host = nullptr;  // pinned mirror
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    std::unique_ptr<hw::HostCopier> copier;  // made by the first large copy into pageable memory
     hw::RedBuf red() const {
         return hw::RedBuf{red_partials.as<double>(), red_ticket.as<unsigned>()};
     }
@@ -176,6 +187,17 @@ int tune_hop(hw_lattice *lat, const hw_gauge *G);
 // (M_s + m_h) on EVEN half fields (d = 1 + m_h), stream-ordered through the lattice's
 // ODD workspace field; context lock held, workspace and hop shape ready
 void eo_apply_half(const hw_gauge *G, double kappa, HalfF64 in, HalfF64 out, int sign, double d);
+// device memory for a force on its way to the host: the context's staging buffer up to
+// kForceStage bytes, else `own`
+constexpr size_t kForceStage = 512u << 20;
+inline int force_buffer(hw_context *ctx, size_t bytes, DevBuf &own, void **out) {
+    const int rc = bytes <= kForceStage ? ensure_stage(ctx, bytes) : own.alloc(bytes);
+    *out = bytes <= kForceStage ? ctx->stage.ptr : own.ptr;
+    return rc;
+}
+// device -> host after the work on the context's stream; returns when dst is complete.  The
+// caller holds the context's lock.
+int copy_to_host(hw_context *ctx, void *dst, const void *src, size_t bytes);
 void destroy_engines(hw_context *ctx);
 
 template <class Body>

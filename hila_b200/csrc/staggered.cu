@@ -409,9 +409,7 @@ int hw_stag_field_download(const hw_stag_field *f, double *host, int parity) {
             k_stag_layout<<<(unsigned)((lat->Vh + 255) / 256), 256, 0, ctx->stream>>>(
                 lat->g, p, ctx->stage.as<double2>(), half_of(f, p), 0);
     HW_CUDA(cudaGetLastError());
-    HW_CUDA(cudaMemcpyAsync(host, ctx->stage.ptr, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    HW_CUDA(cudaStreamSynchronize(ctx->stream));
-    return HW_OK;
+    return copy_to_host(ctx, host, ctx->stage.ptr, bytes);
 }
 
 int hw_stag_field_zero(hw_stag_field *f, int parity) {
@@ -445,24 +443,24 @@ int hw_staggered_evenodd_force(const hw_gauge *gauge, double mass, const hw_stag
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     HW_CUDA(cudaSetDevice(ctx->device));
     const int stride = lat->stride;
-    DevBuf t1, t2, out;
-    if ((rc = t1.alloc((size_t)3 * stride * sizeof(double2))) != HW_OK) return rc;
-    if ((rc = t2.alloc((size_t)3 * stride * sizeof(double2))) != HW_OK) return rc;
-    if ((rc = out.alloc((size_t)36 * lat->V * sizeof(double2))) != HW_OK) return rc;
-    const HalfStag h1{t1.as<double2>(), stride}, h2{t2.as<double2>(), stride}, none{nullptr, 0};
+    if ((rc = ensure_stag_ws(lat)) != HW_OK) return rc;
+    DevBuf own;
+    void *out = nullptr;
+    const size_t bytes = (size_t)36 * lat->V * sizeof(double2);
+    if ((rc = force_buffer(ctx, bytes, own, &out)) != HW_OK) return rc;
+    const HalfStag h1{lat->stag_ws->t.as<double2>(), stride}, h2{lat->stag_ws->Dp[0].as<double2>(), stride},
+        none{nullptr, 0};
     stag_hop_any(gauge, 1, -sign, half_of(chi, 0), none, 0.0, 1.0 / mass, h1, ctx->stream);
     stag_hop_any(gauge, 1, sign, half_of(psi, 0), none, 0.0, 1.0 / mass, h2, ctx->stream);
     dim3 grid((unsigned)((lat->Vh + kStagBlock - 1) / kStagBlock), 2);
     if (sign > 0)
         k_stag_force<1><<<grid, kStagBlock, 0, ctx->stream>>>(lat->g, half_of(chi, 0), half_of(psi, 0), h1, h2,
-                                                              lat->V, out.as<double2>());
+                                                              lat->V, static_cast<double2 *>(out));
     else
         k_stag_force<-1><<<grid, kStagBlock, 0, ctx->stream>>>(lat->g, half_of(chi, 0), half_of(psi, 0), h1, h2,
-                                                               lat->V, out.as<double2>());
+                                                               lat->V, static_cast<double2 *>(out));
     HW_CUDA(cudaGetLastError());
-    HW_CUDA(cudaMemcpyAsync(force, out.ptr, out.bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    HW_CUDA(cudaStreamSynchronize(ctx->stream));
-    return HW_OK;
+    return copy_to_host(ctx, force, out, bytes);
 }
 
 // CG<dirac_staggered_evenodd>::apply (conjugate_gradient.h:46-104): M^dag M out = in

@@ -1008,7 +1008,10 @@ EngGrid eng_grid_size(int low, int variant, int full18, int planes_mask) {
     G.low = sms * lo;
     G.pk = G.low;
     if (variant == 7 && low == LOW_F16) G.pk = sms * occupancy_low<LOW_F16, 2, 3, true, PH_P1>();
-    G.f64 = sms * (hi < 1 ? 1 : hi);
+    // odd: a block's items (k_eng_f64, k_stag_eng) lie this far apart, and with a common factor
+    // with the kEngMaxRhs positions of a tile some blocks met only inactive ones (444 blocks and
+    // one active slot: every fourth block did all the work)
+    G.f64 = (sms * (hi < 1 ? 1 : hi) - 1) | 1;
     int st = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&st, k_stag_low<PH_P4>, kStagLowBlock, 0);
     G.stag = sms * (st < 1 ? 1 : st);

@@ -1013,7 +1013,7 @@ EngGrid eng_grid_size(int low, int variant, int full18, int planes_mask) {
     // one active slot: every fourth block did all the work)
     G.f64 = (sms * (hi < 1 ? 1 : hi) - 1) | 1;
     int st = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&st, k_stag_low<PH_P4>, kStagLowBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&st, k_stag_low<PH_P1>, kStagLowBlock, 0);
     G.stag = sms * (st < 1 ? 1 : st);
     G.kinds = 1;
     G.ntiles = 0;

@@ -139,15 +139,22 @@ __device__ __forceinline__ HalfStag16 stag_low_in(const EngProblem &pr) {
 
 // Own-site operands of a low-precision staggered slot's epilogue, and the epilogue: P1..P5 in
 // FP32 arithmetic on FP16 fields, acc the hop of the slot's input; red[0] receives the
-// phase's |.|^2 contribution.  The operands of two sources are loaded before either is used.
+// phase's |.|^2 contribution.  The operands of a pair are asked for before its hop.
 template <int PHASE>
 struct StagOwn {
-    Cx<float> p[3], r[3], d[3], y[3];
+    uint4 pv, rv, dv;  // as stored, unpacked by finish()
+    float pn, rn, dn;
+    Cx<float> y[3];
     __device__ __forceinline__ void load(const EngProblem &pr, int stride, int i) {
-        if constexpr (PHASE == PH_P2 || PHASE == PH_P4) HalfStag16{static_cast<uint4 *>(pr.p), pr.pn}.ld(i, p);
+        if constexpr (PHASE == PH_P2 || PHASE == PH_P4) {
+            pv = __ldg(static_cast<uint4 *>(pr.p) + i);
+            pn = __ldg(pr.pn + i);
+        }
         if constexpr (PHASE == PH_P4) {
-            HalfStag16{static_cast<uint4 *>(pr.Dp), pr.Dpn}.ld(i, d);
-            HalfStag16{static_cast<uint4 *>(pr.r), pr.rn}.ldp(i, r);
+            dv = __ldg(static_cast<uint4 *>(pr.Dp) + i);
+            dn = __ldg(pr.Dpn + i);
+            rv = static_cast<uint4 *>(pr.r)[i];
+            rn = pr.rn[i];
             const HalfStagY Y{reinterpret_cast<float2 *>(pr.y), stride};
 #pragma unroll
             for (int c = 0; c < 3; c++) y[c] = Y.ld(c, i);
@@ -157,7 +164,12 @@ struct StagOwn {
                                            const Cx<float> (&acc)[3], double *red) {
         constexpr int SIGN = (PHASE == PH_P1 || PHASE == PH_P2) ? 1 : -1;
         const float m = (float)pr.kappa;  // the mass
-        Cx<float> h[3];
+        Cx<float> h[3], p[3], r[3], d[3];
+        if constexpr (PHASE == PH_P2 || PHASE == PH_P4) HalfStag16::unpack(pv, pn, p);
+        if constexpr (PHASE == PH_P4) {
+            HalfStag16::unpack(rv, rn, r);
+            HalfStag16::unpack(dv, dn, d);
+        }
 #pragma unroll
         for (int c = 0; c < 3; c++) h[c] = (0.5f * SIGN) * acc[c];
         if constexpr (PHASE == PH_P1 || PHASE == PH_P3) {  // t = (1/m) D in
@@ -192,7 +204,7 @@ struct StagOwn {
 // shared memory once, the block's teams take the pairs of slots in turn, and each slot's partial
 // sum is formed once per tile in block_sum's order.
 template <int PHASE>
-__global__ void __launch_bounds__(kStagLowBlock, 3) k_stag_low(EngPtrs P) {
+__global__ void __launch_bounds__(kStagLowBlock, PHASE == PH_P4 ? 2 : 3) k_stag_low(EngPtrs P) {
     constexpr int OUTPAR = (PHASE == PH_P1 || PHASE == PH_P3) ? 1 : 0;
     constexpr int NRED = (PHASE == PH_P2 || PHASE == PH_P4) ? 1 : 0;
     __shared__ double smem[kStagLowBlock / 32];
@@ -274,10 +286,10 @@ __global__ void __launch_bounds__(kStagLowBlock, 3) k_stag_low(EngPtrs P) {
             double redA = 0.0, redB = 0.0;
             if (on) {
                 Cx2 acc[3];
-                stag_hop_pair(US, nb, eta, OUTPAR, inA, inB, first, acc);
                 StagOwn<PHASE> oa, ob;
                 oa.load(A, stride, i);
-                if (two) ob.load(B, stride, i);
+                ob.load(B, stride, i);
+                stag_hop_pair(US, nb, eta, OUTPAR, inA, inB, first, acc);
                 Cx<float> ha[3], hb[3];
 #pragma unroll
                 for (int c = 0; c < 3; c++) {

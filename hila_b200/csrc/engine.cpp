@@ -434,9 +434,31 @@ int Engine::build_graph() {
     cudaGraphNode_t wnode;
     HW_CUDA(cudaGraphAddNode(&wnode, g, nodes.data(), nodes.size(), &np));
     cudaGraph_t body = np.conditional.phGraph_out[0];
+    // body: inner phases -> gate -> IF (a reliable update is pending) { R1..R5L } -> P5 -> control.
+    // The seven (with staggered slots fourteen) phases of an update are not launched in the
+    // other iterations, where each returned at once after some 2 us.
+    cudaGraphConditionalHandle ru;
+    HW_CUDA(cudaGraphConditionalHandleCreate(&ru, body, 0, 0));
+    cudaGraphNodeParams ip = {cudaGraphNodeTypeConditional};
+    ip.conditional.handle = ru;
+    ip.conditional.type = cudaGraphCondTypeIf;
+    ip.conditional.size = 1;
     HW_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    eng_enqueue_iteration(low_, ptrs_, grid_, s);
+    eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_INNER);
+    eng_enqueue_gate(ptrs_, ru, s);
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t ndeps = 0;
+    HW_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &ndeps));
+    cudaGraphNode_t inode;
+    HW_CUDA(cudaGraphAddNode(&inode, body, deps, ndeps, &ip));
+    HW_CUDA(cudaStreamUpdateCaptureDependencies(s, &inode, 1, cudaStreamSetCaptureDependencies));
+    eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_P5);
     eng_enqueue_control(ptrs_, kEngMaxProb, 0, cond, 1, s);
+    HW_CUDA(cudaStreamEndCapture(s, &tmp));
+    HW_CUDA(cudaStreamBeginCaptureToGraph(s, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                          cudaStreamCaptureModeThreadLocal));
+    eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_RU);
     HW_CUDA(cudaStreamEndCapture(s, &tmp));
     cudaError_t e = cudaGraphInstantiate(&chunk_exec_, g, 0);
     cudaGraphDestroy(g);

@@ -749,6 +749,9 @@ __global__ void k_eng_control(EngPtrs P, int nprob, int chunk, cudaGraphConditio
     }
 }
 
+// whether the reliable-update phases of this iteration run (the body of a graph's IF node)
+__global__ void k_eng_gate(EngPtrs P, cudaGraphConditionalHandle h) { cudaGraphSetConditional(h, P.ctl[2] ? 1u : 0u); }
+
 __global__ void k_eng_chunk_begin(EngPtrs P) {
     P.ctl[0] = 0;
     for (int k = 0; k < 2 * kEngPhases; k++) P.sched[k] = 0;
@@ -832,10 +835,10 @@ inline void mark(const cudaEvent_t *ev, int k, cudaStream_t s) {
     if (ev) cudaEventRecord(ev[k], s);
 }
 
-// R1..R5L and P5 (phases 4..11), shared by every launch shape of the inner phases;
-// LowRU launches R4L / R5L in the inner phases' shape
+// R1..R5L (phases 4..10), shared by every launch shape of the inner phases; LowRU launches R4L /
+// R5L in the inner phases' shape
 template <int LOW, class LowRU>
-void enqueue_reliable_update(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
+void enqueue_ru(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
     k_eng_vec<PH_R1, LOW><<<G.low, kEngTile, 0, s>>>(P);
     mark(ev, PH_R2, s);
     launch_f64<PH_R2, LOW>(P, G, s);
@@ -849,6 +852,13 @@ void enqueue_reliable_update(const EngPtrs &P, const EngGrid &G, cudaStream_t s,
     launch_f64<PH_R5, LOW>(P, G, s);
     mark(ev, PH_R5L, s);
     LowRU::template launch<PH_R5L>(P, G, s);
+}
+
+// the parts of an iteration after its inner phases
+template <int LOW, class LowRU>
+void enqueue_rest(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev, int parts) {
+    if (parts & ENG_PART_RU) enqueue_ru<LOW, LowRU>(P, G, s, ev);
+    if (!(parts & ENG_PART_P5)) return;
     mark(ev, PH_P5, s);
     k_eng_vec<PH_P5, LOW><<<G.low, kEngTile, 0, s>>>(P);
     mark(ev, kEngPhases, s);
@@ -876,49 +886,55 @@ struct LowShape {
 };
 
 template <int LOW, bool FULL18>
-void enqueue_iteration_t(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
-    mark(ev, 0, s);
-    launch_low<PH_P1, LOW, 1, 6, FULL18>(P, G, G.low, s);
-    mark(ev, 1, s);
-    launch_low<PH_P2, LOW, 1, 6, FULL18>(P, G, G.low, s);
-    mark(ev, 2, s);
-    launch_low<PH_P3, LOW, 1, 6, FULL18>(P, G, G.low, s);
-    mark(ev, 3, s);
-    launch_low<PH_P4, LOW, 1, 6, FULL18>(P, G, G.low, s);
-    mark(ev, 4, s);
-    enqueue_reliable_update<LOW, LowShape<LOW, FULL18>>(P, G, s, ev);
+void enqueue_iteration_t(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev, int parts) {
+    if (parts & ENG_PART_INNER) {
+        mark(ev, 0, s);
+        launch_low<PH_P1, LOW, 1, 6, FULL18>(P, G, G.low, s);
+        mark(ev, 1, s);
+        launch_low<PH_P2, LOW, 1, 6, FULL18>(P, G, G.low, s);
+        mark(ev, 2, s);
+        launch_low<PH_P3, LOW, 1, 6, FULL18>(P, G, G.low, s);
+        mark(ev, 3, s);
+        launch_low<PH_P4, LOW, 1, 6, FULL18>(P, G, G.low, s);
+        mark(ev, 4, s);
+    }
+    enqueue_rest<LOW, LowShape<LOW, FULL18>>(P, G, s, ev, parts);
 }
 
 // P1 and P3 with two solves per thread in packed FP32 (MINB_PK blocks per SM, G.pk
 // blocks), P2, P4 and the reliable update in the shape of variant 2 (G.low blocks)
 template <int LOW, int MINB_PK, bool FULL18>
-void enqueue_iteration_hybrid(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
-    mark(ev, 0, s);
-    launch_low<PH_P1, LOW, 2, MINB_PK, FULL18, true>(P, G, G.pk, s);
-    mark(ev, 1, s);
-    launch_low<PH_P2, LOW, 1, 6, FULL18>(P, G, G.low, s);
-    mark(ev, 2, s);
-    launch_low<PH_P3, LOW, 2, MINB_PK, FULL18, true>(P, G, G.pk, s);
-    mark(ev, 3, s);
-    launch_low<PH_P4, LOW, 1, 6, FULL18>(P, G, G.low, s);
-    mark(ev, 4, s);
-    enqueue_reliable_update<LOW, LowShape<LOW, FULL18>>(P, G, s, ev);
+void enqueue_iteration_hybrid(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev, int parts) {
+    if (parts & ENG_PART_INNER) {
+        mark(ev, 0, s);
+        launch_low<PH_P1, LOW, 2, MINB_PK, FULL18, true>(P, G, G.pk, s);
+        mark(ev, 1, s);
+        launch_low<PH_P2, LOW, 1, 6, FULL18>(P, G, G.low, s);
+        mark(ev, 2, s);
+        launch_low<PH_P3, LOW, 2, MINB_PK, FULL18, true>(P, G, G.pk, s);
+        mark(ev, 3, s);
+        launch_low<PH_P4, LOW, 1, 6, FULL18>(P, G, G.low, s);
+        mark(ev, 4, s);
+    }
+    enqueue_rest<LOW, LowShape<LOW, FULL18>>(P, G, s, ev, parts);
 }
 
 constexpr int kMmaMinBlocks = 4;
 
 // FP16 inner phases on the tensor cores (engine_mma.cuh), the rest as usual
-void enqueue_iteration_mma(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
-    mark(ev, 0, s);
-    k_eng_mma<PH_P1, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
-    mark(ev, 1, s);
-    k_eng_mma<PH_P2, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
-    mark(ev, 2, s);
-    k_eng_mma<PH_P3, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
-    mark(ev, 3, s);
-    k_eng_mma<PH_P4, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
-    mark(ev, 4, s);
-    enqueue_reliable_update<LOW_F16, LowShape<LOW_F16, true>>(P, G, s, ev);
+void enqueue_iteration_mma(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev, int parts) {
+    if (parts & ENG_PART_INNER) {
+        mark(ev, 0, s);
+        k_eng_mma<PH_P1, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
+        mark(ev, 1, s);
+        k_eng_mma<PH_P2, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
+        mark(ev, 2, s);
+        k_eng_mma<PH_P3, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
+        mark(ev, 3, s);
+        k_eng_mma<PH_P4, kMmaMinBlocks><<<G.low, kEngTile, 0, s>>>(P);
+        mark(ev, 4, s);
+    }
+    enqueue_rest<LOW_F16, LowShape<LOW_F16, true>>(P, G, s, ev, parts);
 }
 
 // Launch shapes of the low-precision phases (EngGrid::variant):
@@ -933,40 +949,43 @@ void enqueue_iteration_mma(const EngPtrs &P, const EngGrid &G, cudaStream_t s, c
 // without packing, packed P1..P4, packed P1..P3, and P1/P3 streaming their neighbour data
 // through a cp.async ring in shared memory were measured slower or no faster and removed)
 template <int LOW, bool FULL18>
-void enqueue_iteration_v(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
+void enqueue_iteration_v(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev, int parts) {
     if constexpr (LOW == LOW_F16) {
         if (G.variant == 4) {
-            enqueue_iteration_mma(P, G, s, ev);
+            enqueue_iteration_mma(P, G, s, ev, parts);
             return;
         }
         if (G.variant == 7) {
-            enqueue_iteration_hybrid<LOW, 3, FULL18>(P, G, s, ev);
+            enqueue_iteration_hybrid<LOW, 3, FULL18>(P, G, s, ev, parts);
             return;
         }
     }
-    enqueue_iteration_t<LOW, FULL18>(P, G, s, ev);
+    enqueue_iteration_t<LOW, FULL18>(P, G, s, ev, parts);
 }
 
 template <int LOW>
-void enqueue_iteration_nr(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
+void enqueue_iteration_nr(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev, int parts) {
     if (G.full18)
-        enqueue_iteration_v<LOW, true>(P, G, s, ev);
+        enqueue_iteration_v<LOW, true>(P, G, s, ev, parts);
     else
-        enqueue_iteration_v<LOW, false>(P, G, s, ev);
+        enqueue_iteration_v<LOW, false>(P, G, s, ev, parts);
 }
 
 }  // namespace
 
-void eng_enqueue_iteration(int low, const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev) {
+void eng_enqueue_iteration(int low, const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cudaEvent_t *ev,
+                           int parts) {
     if (G.kinds & 1) {
         if (low == LOW_F16)
-            enqueue_iteration_nr<LOW_F16>(P, G, s, ev);
+            enqueue_iteration_nr<LOW_F16>(P, G, s, ev, parts);
         else
-            enqueue_iteration_nr<LOW_F32>(P, G, s, ev);
+            enqueue_iteration_nr<LOW_F32>(P, G, s, ev, parts);
     }
     // staggered phases after the Wilson ones (outside the profiling events)
-    if (G.kinds & 6) enqueue_stag_iteration(P, G, s);
+    if (G.kinds & 6) enqueue_stag_iteration(P, G, s, parts);
 }
+
+void eng_enqueue_gate(const EngPtrs &P, cudaGraphConditionalHandle h, cudaStream_t s) { k_eng_gate<<<1, 1, 0, s>>>(P, h); }
 
 void eng_enqueue_control(const EngPtrs &P, int nprob, int chunk, cudaGraphConditionalHandle h, int use_cond,
                          cudaStream_t s) {

@@ -168,10 +168,14 @@ __host__ __device__ constexpr bool eng_ru_phase(int ph) { return ph >= PH_R1 && 
 // low-precision format of one engine (template parameter of the inner phases)
 enum EngLow : int { LOW_F32 = 1, LOW_F16 = 2 };
 
-// Enqueue one CG iteration (all phases) on stream s.  With ev (kEngPhases + 1
+// parts of an iteration, in order
+enum EngPart : int { ENG_PART_INNER = 1, ENG_PART_RU = 2, ENG_PART_P5 = 4, ENG_PART_ALL = 7 };
+// Enqueue one CG iteration (or some of its parts) on stream s.  With ev (kEngPhases + 1
 // events) ev[k] is recorded before phase k and ev[kEngPhases] after the last.
 void eng_enqueue_iteration(int low, const EngPtrs &P, const EngGrid &G, cudaStream_t s,
-                           const cudaEvent_t *ev = nullptr);
+                           const cudaEvent_t *ev = nullptr, int parts = ENG_PART_ALL);
+// Sets the handle of a graph's IF node by whether some slot asked for a reliable update.
+void eng_enqueue_gate(const EngPtrs &P, cudaGraphConditionalHandle h, cudaStream_t s);
 // While-loop control: counts running slots, stops after `chunk` iterations or when none runs.
 void eng_enqueue_control(const EngPtrs &P, int nprob, int chunk, cudaGraphConditionalHandle h, int use_cond,
                          cudaStream_t s);

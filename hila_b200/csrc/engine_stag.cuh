@@ -202,7 +202,10 @@ struct StagOwn {
 // P1..P4 of the staggered slots with FP16 inner iterations: a block takes items (a tile and a
 // part of its slots) from a counter; per item, the sites' eight FP16 links are copied into
 // shared memory once, the block's teams take the pairs of slots in turn, and each slot's partial
-// sum is formed once per tile in block_sum's order.
+// sum is formed once per tile in block_sum's order.  Bound by load latency: at 24^4 with 8
+// sources P1 takes 54 us (100 MB: 15 us at the HBM's rate), P2 80, P4 98; one source a thread
+// with 16 warps per SM took 62, 92 and 132.  P4 holds its pair's own-site operands during the
+// hop, in 128 registers (24 warps with 80 registers: 111 us); P2 is slower that way (84 us).
 template <int PHASE>
 __global__ void __launch_bounds__(kStagLowBlock, PHASE == PH_P4 ? 2 : 3) k_stag_low(EngPtrs P) {
     constexpr int OUTPAR = (PHASE == PH_P1 || PHASE == PH_P3) ? 1 : 0;
@@ -534,23 +537,29 @@ __global__ void __launch_bounds__(kEngTile, 3) k_stag_eng(EngPtrs P) {
 // one iteration of the staggered slots: the phases of the slot kinds present (FP64 and FP16
 // slots of a phase are disjoint; each kernel finishes its own); the reliable-update phases,
 // which serve both kinds, return at once unless some slot asked for one
-void enqueue_stag_iteration(const EngPtrs &P, const EngGrid &G, cudaStream_t s) {
+void enqueue_stag_iteration(const EngPtrs &P, const EngGrid &G, cudaStream_t s, int parts) {
     const bool f64 = G.kinds & 2, low = G.kinds & 4;
-    if (f64) k_stag_eng<PH_P1><<<G.f64, kEngTile, 0, s>>>(P);
-    if (low) k_stag_low<PH_P1><<<G.stag, kStagLowBlock, 0, s>>>(P);
-    if (f64) k_stag_eng<PH_P2><<<G.f64, kEngTile, 0, s>>>(P);
-    if (low) k_stag_low<PH_P2><<<G.stag, kStagLowBlock, 0, s>>>(P);
-    if (f64) k_stag_eng<PH_P3><<<G.f64, kEngTile, 0, s>>>(P);
-    if (low) k_stag_low<PH_P3><<<G.stag, kStagLowBlock, 0, s>>>(P);
-    if (f64) k_stag_eng<PH_P4><<<G.f64, kEngTile, 0, s>>>(P);
-    if (low) k_stag_low<PH_P4><<<G.stag, kStagLowBlock, 0, s>>>(P);
-    k_stag_eng<PH_R1><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_R2><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_R3><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_R4><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_R4L><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_R5><<<G.f64, kEngTile, 0, s>>>(P);
-    k_stag_eng<PH_R5L><<<G.f64, kEngTile, 0, s>>>(P);
-    if (f64) k_stag_eng<PH_P5><<<G.f64, kEngTile, 0, s>>>(P);
-    if (low) k_stag_low_p5<<<4 * G.stag, kEngTile, 0, s>>>(P);
+    if (parts & ENG_PART_INNER) {
+        if (f64) k_stag_eng<PH_P1><<<G.f64, kEngTile, 0, s>>>(P);
+        if (low) k_stag_low<PH_P1><<<G.stag, kStagLowBlock, 0, s>>>(P);
+        if (f64) k_stag_eng<PH_P2><<<G.f64, kEngTile, 0, s>>>(P);
+        if (low) k_stag_low<PH_P2><<<G.stag, kStagLowBlock, 0, s>>>(P);
+        if (f64) k_stag_eng<PH_P3><<<G.f64, kEngTile, 0, s>>>(P);
+        if (low) k_stag_low<PH_P3><<<G.stag, kStagLowBlock, 0, s>>>(P);
+        if (f64) k_stag_eng<PH_P4><<<G.f64, kEngTile, 0, s>>>(P);
+        if (low) k_stag_low<PH_P4><<<G.stag, kStagLowBlock, 0, s>>>(P);
+    }
+    if (parts & ENG_PART_RU) {
+        k_stag_eng<PH_R1><<<G.f64, kEngTile, 0, s>>>(P);
+        k_stag_eng<PH_R2><<<G.f64, kEngTile, 0, s>>>(P);
+        k_stag_eng<PH_R3><<<G.f64, kEngTile, 0, s>>>(P);
+        k_stag_eng<PH_R4><<<G.f64, kEngTile, 0, s>>>(P);
+        k_stag_eng<PH_R4L><<<G.f64, kEngTile, 0, s>>>(P);
+        k_stag_eng<PH_R5><<<G.f64, kEngTile, 0, s>>>(P);
+        k_stag_eng<PH_R5L><<<G.f64, kEngTile, 0, s>>>(P);
+    }
+    if (parts & ENG_PART_P5) {
+        if (f64) k_stag_eng<PH_P5><<<G.f64, kEngTile, 0, s>>>(P);
+        if (low) k_stag_low_p5<<<4 * G.stag, kEngTile, 0, s>>>(P);
+    }
 }

@@ -25,9 +25,9 @@ void fill_result(const EngState &s, double seconds, int chunks, hw_cg_result *R)
     R->rr_relative = s.b2 > 0 ? s.rr / s.b2 : 0.0;
     R->true_residual = s.b2 > 0 ? std::sqrt(s.s2 / s.b2) : 0.0;
     R->seconds = seconds;
-    // every loop body launches 10 phase kernels and one control kernel; the
-    // first body of a slot is its initial residual (no inner iteration)
-    R->kernel_launches = chunks + 11 * (s.iter + 1);
+    // every loop body launches P1..P4, the gate, P5 and the control kernel, a body with a
+    // reliable update its seven phases more; every chunk one kernel
+    R->kernel_launches = chunks + 7 * (s.iter + 1) + 7 * s.n_ru;
     if (s.status == ENG_CONVERGED)
         R->status = HW_OK;
     else if (s.status == ENG_BREAKDOWN)

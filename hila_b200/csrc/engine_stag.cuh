@@ -6,10 +6,10 @@
 //
 // The operator is dirac_staggered_evenodd (staggered.h:193-279) as the reference codes
 // it: M_s in = m in_e + D^{eo}_s (1/m) D^{oe}_s in_e with D_s = 0.5 s hop, M^dag = M_{-s}.
-// Everything runs in FP64 (the colour vector is small, the phases are bound by memory
-// and latency); the low-precision buffers of a slot hold FP64 half lattices here (3
-// double2 planes: 48 bytes per site, the size of a Wilson FP16 buffer).  Work items are
-// (tile, active slot) pairs as in the Wilson FP64 phases.  The site algebra comes from
+// FP64 slots run in FP64 throughout, in k_stag_eng: the low-precision buffers of a slot hold
+// FP64 half lattices (3 double2 planes: 48 bytes per site, the size of a Wilson FP16 buffer)
+// and work items are (tile, active slot) pairs as in the Wilson FP64 phases.  Slots with FP16
+// inner iterations run P1..P5 in k_stag_low and share k_stag_eng's reliable update.  The site algebra comes from
 // staggered_math.cuh, which engine.cu includes at file scope.
 #pragma once
 

@@ -10,11 +10,10 @@
 //   K4  DDp  = Dp - kappa^2 H^{eo}_- t; x += alpha p; r -= alpha DDp
 //                                             + |r|^2 -> beta, convergence
 //   P   p    = r + beta p, and the loop's condition
-// alpha, beta and the stopping
-// decision stay in device memory.  The body is captured into the body graph
-// of a CUDA-graph WHILE node, so a whole solve is one graph launch and one
-// host synchronisation; the explicit FP64 residual check is appended to the
-// same graph.
+// alpha, beta and the stopping decision stay in device memory.  The body is
+// captured into the body graph of a CUDA-graph WHILE node, so a whole solve is
+// one graph launch and one host synchronisation; the explicit FP64 residual
+// check is appended to the same graph.
 #include <cuda_runtime.h>
 
 #include <cmath>

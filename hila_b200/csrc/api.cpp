@@ -114,9 +114,10 @@ int ensure_stage(hw_context *ctx, size_t bytes) {
 }
 
 int ensure_reduction_capacity(hw_context *ctx, long nblocks) {
-    size_t need = (size_t)4 * (nblocks + 1);
+    const size_t need = red_doubles(nblocks);
     if (ctx->red_capacity_doubles >= need) return HW_OK;
     HW_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->red_capacity_doubles = 0;  // the old buffer is gone if the new one cannot be had
     int rc = ctx->red_partials.alloc(need * sizeof(double));
     if (rc != HW_OK) return rc;
     ctx->red_capacity_doubles = need;

@@ -301,7 +301,6 @@ __device__ __forceinline__ Cx<double> add_phase(Cx<double> acc, Cx<double> v) {
     return acc - mul_i(v);
 }
 
-constexpr int kSplitSites = 32;                 // sites of a block: one per lane
 constexpr int kSplitBlock = 8 * kSplitSites;    // a warp per term of the hop
 using SplitTerms = double2[8][6][kSplitSites];  // [term][3 * half spinor + colour][site]
 
@@ -384,10 +383,16 @@ __global__ void __launch_bounds__(kSplitBlock, 2) k_hop_split(Geom g, Lk U, int 
     if constexpr (Epi::NRED > 0) grid_reduce<Epi::NRED, kSplitBlock>(v, red.partials, red.ticket, epi);
 }
 
+template <class Epi>
+dim3 hop_grid(int variant, const Geom &g, const RedBuf &rb) {
+    const long nb = hop_blocks(variant, g.Vh);
+    return Epi::NRED > 0 ? rb.grid(Epi::NRED, nb) : dim3((unsigned)nb);
+}
+
 template <class Lk, class Epi>
 void launch_split(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin, const Epi &epi, RedBuf rb,
                   cudaStream_t s) {
-    dim3 grid((g.Vh + kSplitSites - 1) / kSplitSites);
+    const dim3 grid = hop_grid<Epi>(3, g, rb);
     if (sign > 0)
         launch_chain(g.chain, k_hop_split<1, Lk, Epi>, grid, kSplitBlock, 0, s, g, L, par, sin, epi, rb);
     else
@@ -419,7 +424,8 @@ size_t hop_smem() {
 template <int BLOCK, int MINB, class Lk, class Epi>
 void launch_variant(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin, const Epi &epi, RedBuf rb,
                     cudaStream_t s) {
-    dim3 grid((g.Vh + BLOCK - 1) / BLOCK);
+    const dim3 grid = hop_grid<Epi>(BLOCK == 256 ? 2 : 0, g, rb);
+    static_assert(hop_sites(BLOCK == 256 ? 2 : 0) == BLOCK, "shape and block size");
     if (sign > 0)
         launch_chain(g.chain, k_hop<1, BLOCK, MINB, Lk, Epi>, grid, BLOCK, hop_smem<1, BLOCK, MINB, Lk, Epi>(), s, g, L,
                      par, sin, epi, rb);
@@ -428,7 +434,7 @@ void launch_variant(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin
                      par, sin, epi, rb);
 }
 
-// Launch shapes the autotuner chooses from (HopVariant in kernels.h):
+// Launch shapes the autotuner chooses from (hop_shapes.h):
 //   0: 128 threads, registers unconstrained   1: 128 threads, <= 128 registers (4 blocks/SM)
 //   2: 256 threads, <= 128 registers
 // and, not timed, 3: k_hop_split, for lattices up to kHopSplitSites
@@ -456,7 +462,7 @@ void launch_shape(const Geom &g, const Lk &L, int par, int sign, SpinorF64 sin, 
 template <class Epi>
 void dispatch_hop(const Geom &g, const GaugeF64 &U, int par, int sign, HalfF64 in, const Epi &epi, const RedBuf *red,
                   cudaStream_t s) {
-    RedBuf rb = red ? *red : RedBuf{nullptr, nullptr};
+    RedBuf rb = red ? *red : RedBuf{nullptr, nullptr, 0};
     SpinorF64 sin{in.p, in.stride};
     if (U.planes == 9)
         launch_shape(g, LinksF64x18{U.p, U.stride}, par, sign, sin, epi, rb, s);
@@ -647,8 +653,8 @@ void launch_hop_residual(const Geom &g, const GaugeF64 &U, int par, int sign, Ha
 void launch_cg_init(int Vh, HalfF64 src, HalfF64 Ax, HalfF64 r, HalfF64 p, double acc2, int maxiter, CgState *st,
                     const RedBuf &red, cudaStream_t s) {
     FinCgInit fin{st, acc2, maxiter};
-    k_cg_init<<<(Vh + kVecBlock - 1) / kVecBlock, kVecBlock, 0, s>>>(Vh, sp(src), sp(Ax), Ax.p != nullptr, sp(r),
-                                                                      sp(p), fin, red);
+    k_cg_init<<<red.grid(2, (Vh + kVecBlock - 1) / kVecBlock), kVecBlock, 0, s>>>(Vh, sp(src), sp(Ax), Ax.p != nullptr,
+                                                                                  sp(r), sp(p), fin, red);
 }
 
 void launch_cg_pupdate(int Vh, HalfF64 r, HalfF64 p, CgState *st, cudaGraphConditionalHandle cond, int use_cond,

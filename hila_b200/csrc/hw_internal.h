@@ -85,7 +85,7 @@ struct hw_context {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::unique_ptr<hw::HostCopier> copier;  // made by the first large copy into pageable memory
     hw::RedBuf red() const {
-        return hw::RedBuf{red_partials.as<double>(), red_ticket.as<unsigned>()};
+        return hw::RedBuf{red_partials.as<double>(), red_ticket.as<unsigned>(), red_capacity_doubles};
     }
     size_t red_capacity_doubles = 0;
     hw::Engine *engines[3] = {nullptr, nullptr, nullptr};  // batched mixed-precision engines by precision

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "hop_shapes.h"
 #include "wilson_math.cuh"
 
 namespace hw {
@@ -48,14 +49,6 @@ __device__ __forceinline__ T *chained(T *p) {
 }
 #endif
 
-constexpr int kHopBlock = 128;
-constexpr int kHopMinBlock = 128;  // smallest block of any hop launch shape (sizes reduction buffers)
-constexpr int kHopVariants = 4;  // 0..2 timed per lattice, 3 for small lattices (dslash_f64.cu)
-// Sites per parity up to which the hop runs eight warps per 32 sites (k_hop_split): an FP64 CG
-// iteration took 40 -> 30 us at 8^4, 43 -> 39 us at 6x10x14x22 (9240), 43 -> 44 us at 12^4
-// (10368), 52 -> 65 us at 16^4.
-constexpr int kHopSplitSites = 9500;
-
 // Device-resident scalars of one FP64 conjugate-gradient solve
 // (conjugate_gradient.h:55-57 keeps the same quantities on the host).
 struct CgState {
@@ -83,8 +76,14 @@ __device__ __forceinline__ void loop_next(const CgState *st, cudaGraphConditiona
 
 // Work buffers for one grid reduction: partial sums and the arrival ticket.
 struct RedBuf {
-    double *partials;  // >= 4 * max blocks
+    double *partials;
     unsigned *ticket;  // one counter, zero between uses
+    size_t capacity;   // doubles that partials holds
+    // the grid of a reducing launch: the one asked for if its partial sums fit, else an empty
+    // one, which the launch refuses (cudaErrorInvalidConfiguration)
+    dim3 grid(int nred, long nblocks) const {
+        return dim3((size_t)nred * nblocks <= capacity ? (unsigned)nblocks : 0u);
+    }
 };
 
 // FP64 spinor half-lattice: 12 double2 planes

@@ -76,7 +76,7 @@ struct Mre {
     int blocks;
 
     void rdot(HalfF64 a, HalfF64 b, double *out) {
-        k_rdot<<<blocks, kMreBlock, 0, ctx->stream>>>(Vh, a, b, StoreSum{out}, ctx->red());
+        k_rdot<<<ctx->red().grid(1, blocks), kMreBlock, 0, ctx->stream>>>(Vh, a, b, StoreSum{out}, ctx->red());
     }
     void project_out(const double *ov, const double *n2, HalfF64 x, HalfF64 y) {
         k_project_out<<<blocks, kMreBlock, 0, ctx->stream>>>(Vh, ov, n2, x, y);

@@ -136,7 +136,7 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
     const double acc2 = P.accuracy * P.accuracy;
     const int use_graph = P.use_graph;
     int rc;
-    if ((rc = ensure_reduction_capacity(ctx, (S.lat->Vh + kHopBlock - 1) / kHopBlock)) != HW_OK) return rc;
+    if ((rc = ensure_reduction_capacity(ctx, hop_blocks(S.lat->g.hop_variant, S.lat->Vh))) != HW_OK) return rc;
     S.red = ctx->red();
 
     CgWorkspace::Key key;

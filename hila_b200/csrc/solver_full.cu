@@ -186,19 +186,20 @@ template <class Epi>
 void full_hop(const hw_gauge *G, int sign, Full in, const Epi &epi, RedBuf red, cudaStream_t s) {
     const Geom &g = G->lat->g;
     const GaugeF64 U = G->U();
-    const int nb = 2 * ((g.Vh + kFullBlock - 1) / kFullBlock);
+    const long nb = 2L * ((g.Vh + kFullBlock - 1) / kFullBlock);
+    const dim3 grid = Epi::NRED > 0 ? red.grid(Epi::NRED, nb) : dim3((unsigned)nb);
     const LinksF64x18 U18{U.p, U.stride};
     const LinksF64x12 U12{U.p, U.stride};
     if (U.planes == 9) {
         if (sign > 0)
-            k_full_hop<1><<<nb, kFullBlock, 0, s>>>(g, U18, in, epi, red);
+            k_full_hop<1><<<grid, kFullBlock, 0, s>>>(g, U18, in, epi, red);
         else
-            k_full_hop<-1><<<nb, kFullBlock, 0, s>>>(g, U18, in, epi, red);
+            k_full_hop<-1><<<grid, kFullBlock, 0, s>>>(g, U18, in, epi, red);
     } else {
         if (sign > 0)
-            k_full_hop<1><<<nb, kFullBlock, 0, s>>>(g, U12, in, epi, red);
+            k_full_hop<1><<<grid, kFullBlock, 0, s>>>(g, U12, in, epi, red);
         else
-            k_full_hop<-1><<<nb, kFullBlock, 0, s>>>(g, U12, in, epi, red);
+            k_full_hop<-1><<<grid, kFullBlock, 0, s>>>(g, U12, in, epi, red);
     }
 }
 

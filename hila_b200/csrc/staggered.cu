@@ -254,19 +254,20 @@ template <class Epi>
 void stag_cg(const hw_gauge *G, int par, int sign, HalfStag in, const Epi &epi, RedBuf red, cudaStream_t s) {
     const GaugeF64 U = G->U();
     const Geom &g = G->lat->g;
-    const int nb = (g.Vh + kStagBlock - 1) / kStagBlock;
+    const long nb = (g.Vh + kStagBlock - 1) / kStagBlock;
+    const dim3 grid = Epi::NRED > 0 ? red.grid(Epi::NRED, nb) : dim3((unsigned)nb);
     const LinksF64x18 U18{U.p, U.stride};
     const LinksF64x12 U12{U.p, U.stride};
     if (U.planes == 9) {
         if (sign > 0)
-            k_stag_cg<1><<<nb, kStagBlock, 0, s>>>(g, U18, par, in, epi, red);
+            k_stag_cg<1><<<grid, kStagBlock, 0, s>>>(g, U18, par, in, epi, red);
         else
-            k_stag_cg<-1><<<nb, kStagBlock, 0, s>>>(g, U18, par, in, epi, red);
+            k_stag_cg<-1><<<grid, kStagBlock, 0, s>>>(g, U18, par, in, epi, red);
     } else {
         if (sign > 0)
-            k_stag_cg<1><<<nb, kStagBlock, 0, s>>>(g, U12, par, in, epi, red);
+            k_stag_cg<1><<<grid, kStagBlock, 0, s>>>(g, U12, par, in, epi, red);
         else
-            k_stag_cg<-1><<<nb, kStagBlock, 0, s>>>(g, U12, par, in, epi, red);
+            k_stag_cg<-1><<<grid, kStagBlock, 0, s>>>(g, U12, par, in, epi, red);
     }
 }
 

@@ -108,3 +108,18 @@ def test_loop_graph_solvers(hw, ctx, oracle, dims, link_format):
             S.apply(sx, sy)
             S.dagger(sy, sz)
             assert rel(sz.download(hw.EVEN), sb.download(hw.EVEN)) <= 10 * ACC
+
+
+@pytest.mark.parametrize("variant", ["0", "1", "2", "3"])
+def test_every_hop_shape(hw, ctx, oracle, monkeypatch, variant):
+    """Each launch shape on a lattice above the limit of the small lattices' rule (10368 sites per
+    parity): the sums of an explicit residual fit the buffer reserved for that shape."""
+    dims = (12, 12, 12, 12)
+    monkeypatch.setenv("HW_HOP_VARIANT", variant)
+    lat = hw.Lattice(ctx, dims)
+    D = hw.Dirac_Wilson_evenodd(0.12, hw.GaugeField(lat, oracle.gen_links(dims, 0.3, 5)))
+    b, x, y = hw.Field(lat, oracle.gen_spinor(dims, 6, oracle.EVEN)), hw.Field(lat), hw.Field(lat)
+    r = D.solve(b, x, accuracy=ACC)
+    assert r.converged and r.true_residual <= ACC
+    D.apply(x, y)
+    assert rel(y.download(), b.download()) <= 2 * ACC

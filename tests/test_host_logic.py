@@ -1,0 +1,23 @@
+"""Host-side logic that needs no GPU, compiled and run on the CPU: the sizes of the grid
+reductions (hila_b200/csrc/hop_shapes.h) by tests/cpp/test_reductions.cpp."""
+import os
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "hila_b200", "csrc")
+
+
+def compile_and_run(tmp_path, name, *flags):
+    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    exe = str(tmp_path / name)
+    cc = subprocess.run([cxx, "-std=c++17", "-O2", "-Wall", "-Werror", "-I", CSRC,
+                         os.path.join(ROOT, "tests", "cpp", name + ".cpp"), *flags, "-o", exe],
+                        capture_output=True, text=True)
+    assert cc.returncode == 0, cc.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
+
+
+def test_reduction_sizes(tmp_path):
+    assert "reduction sizes passed" in compile_and_run(tmp_path, "test_reductions")

@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "cg_loop.cuh"
 #include "hw_internal.h"
 #include "reduce.cuh"
 #include "storage.cuh"
@@ -54,23 +55,9 @@ struct FullMul {
         red[0] = n2;
     }
     __device__ void operator()(const double *tot) {
-        st->pAp = tot[0];
-        if (!(tot[0] > 0.0) || !isfinite(tot[0]))
-            st->status = CG_BREAKDOWN, st->do_pupdate = 0;
-        else
-            st->alpha = st->rr / tot[0];
+        cg_alpha(st, tot[0]);
     }
 };
-
-// the status after |r|^2 = rr, as conjugate_gradient.h:66-69 loops: while rr >= target
-__device__ __forceinline__ void full_status(CgState *st) {
-    if (!(st->rr >= st->target_rr))
-        st->status = CG_CONVERGED;
-    else if (st->iter >= st->maxiter)
-        st->status = CG_MAXITER;
-    else
-        st->status = CG_RUNNING;
-}
 
 // r = p = b - (Dp - k H Dp); |r|^2, |b|^2 -> the start of the iteration
 struct FullInit {
@@ -92,15 +79,7 @@ struct FullInit {
         }
     }
     __device__ void operator()(const double *tot) {
-        st->rr = tot[0];
-        st->src_norm2 = tot[1];
-        st->target_rr = acc2 * tot[1];
-        st->iter = 0;
-        st->maxiter = maxiter;
-        st->alpha = st->beta = 0.0;
-        st->do_pupdate = 0;
-        full_status(st);
-        if (!(tot[1] > 0.0)) st->status = CG_CONVERGED;
+        cg_start(st, tot[0], tot[1], acc2, maxiter);
     }
 };
 
@@ -125,11 +104,7 @@ struct FullUpdate {
         red[0] = n2;
     }
     __device__ void operator()(const double *tot) {
-        st->iter += 1;
-        st->beta = tot[0] / st->rr;
-        st->rr = tot[0];
-        st->do_pupdate = 1;
-        full_status(st);
+        cg_step(st, tot[0]);
     }
 };
 
@@ -279,7 +254,8 @@ extern "C" int hw_wilson_cg_solve(const hw_gauge *gauge, double kappa, const hw_
     int status = h->status == CG_BREAKDOWN ? HW_ERR_BREAKDOWN
                  : h->status == CG_MAXITER ? HW_ERR_NOT_CONVERGED
                                            : HW_OK;
-    if (status == HW_OK && P.true_residual && true_res > P.accuracy) status = HW_ERR_NOT_CONVERGED;
+    if (status == HW_OK && (!std::isfinite(true_res) || (P.true_residual && true_res > P.accuracy)))
+        status = HW_ERR_NOT_CONVERGED;
     if (result) {
         std::memset(result, 0, sizeof(*result));
         float ms = 0.f;

@@ -123,3 +123,40 @@ def test_every_hop_shape(hw, ctx, oracle, monkeypatch, variant):
     assert r.converged and r.true_residual <= ACC
     D.apply(x, y)
     assert rel(y.download(), b.download()) <= 2 * ACC
+
+
+@pytest.mark.parametrize("kind", ["wilson", "staggered"])
+def test_loop_graph_limits(hw, ctx, oracle, kind):
+    """The loop-graph solvers on a source or guess that is not finite (a breakdown, as in the
+    even-odd CG), at an iteration limit, on a zero source, and on a good source afterwards."""
+    dims = (4, 6, 2, 8)
+    lat = hw.Lattice(ctx, dims)
+    G = hw.GaugeField(lat, oracle.gen_links(dims, 0.3, 5))
+    op = hw.Dirac_Wilson(0.11, G) if kind == "wilson" else hw.dirac_staggered_evenodd(4.0, G)
+    comps = (4, 3, 2) if kind == "wilson" else (3, 2)
+    good = np.random.default_rng(3).standard_normal((lat.volume, *comps))
+
+    def field(host):
+        return hw.Field(lat, host) if kind == "wilson" else hw.StaggeredField(lat, host, hw.EVEN)
+
+    def solve(b, x, **kw):
+        fb, fx = field(b), field(x)
+        r = op.cg(fb, fx, accuracy=1e-10, **kw)
+        return r, fx.download(hw.ALL if kind == "wilson" else hw.EVEN)
+
+    zero = np.zeros_like(good)
+    for value in (np.nan, np.inf, 1e200):  # the square of the last overflows
+        for site in ((0, lat.volume - 1) if kind == "wilson" else (0,)):
+            bad = good.copy()
+            bad[(site,) + (0,) * len(comps)] = value
+            for true_residual in (False, True):
+                r, _ = solve(bad, zero, true_residual=true_residual)
+                assert r.status == hw.HW_ERR_BREAKDOWN and r.iterations == 0
+                r, _ = solve(good, bad, true_residual=true_residual)
+                assert r.status == hw.HW_ERR_BREAKDOWN and r.iterations == 0
+    r, _ = solve(good, zero, maxiters=3)
+    assert r.status == hw.HW_ERR_NOT_CONVERGED and r.iterations == 3
+    r, x = solve(zero, zero)
+    assert r.converged and r.iterations == 0 and not x.any()
+    r, _ = solve(good, zero, true_residual=True)
+    assert r.converged and r.true_residual <= 1e-10

@@ -7,6 +7,7 @@
 #include <cstring>
 
 #include "engine_host.h"
+#include "engine_parts.h"
 
 namespace hw {
 
@@ -171,6 +172,8 @@ int Engine::prune_lattices() {
     EngTables nt;
     std::memset(&nt, 0, sizeof(nt));
     nt.dyn = tables_.dyn;
+    std::memcpy(nt.parts, tables_.parts, sizeof(nt.parts));
+    std::memcpy(nt.even, tables_.even, sizeof(nt.even));
     std::vector<const hw_gauge *> ng;
     std::vector<int> remap(tables_.nlat, -1);
     for (int l : keep) {
@@ -466,6 +469,25 @@ int Engine::build_graph() {
     return HW_OK;
 }
 
+// The parts of the tiles (engine_parts.h) for the slots and the launch grids of the next chunk.
+void Engine::divide_tiles() {
+    const int overhead = low_ == LOW_F16 ? kPartsOverheadF16 : kPartsOverheadF32;
+    const PartsShape shapes[kEngItemKinds] = {
+        {grid_.low, 1, 1, overhead}, {grid_.pk, 2, 1, kPartsOverheadPair}, {grid_.stag, 2, 2, kPartsOverheadPair}};
+    for (int k = 0; k < kEngItemKinds; k++) {
+        const int fermion = k == ITEMS_STAG ? FERM_STAGGERED : FERM_WILSON;
+        PartsLattice lat[kEngMaxLat];
+        for (int l = 0; l < tables_.nlat; l++)
+            lat[l] = {tables_.lat[l].ntiles, tables_.lat[l].fermion == fermion ? tables_.lat[l].nprob : 0};
+        const int parts = choose_parts(lat, tables_.nlat, shapes[k], kEngMaxRhs);
+        const int even = parts_even(lat, tables_.nlat, shapes[k], parts);
+        if (tables_.parts[k] != parts || tables_.even[k] != even) tables_dirty_ = true;
+        tables_.parts[k] = parts;
+        tables_.even[k] = even;
+        grid_.divided[k] = parts > 1;
+    }
+}
+
 int Engine::configure() {
     int mask = 0, kinds = 0;
     for (int l = 0; l < tables_.nlat; l++) mask |= tables_.lat[l].l64_planes == 9 ? 1 : 2;
@@ -487,14 +509,15 @@ int Engine::configure() {
     const bool known =
         variant == 2 || (low_ == LOW_F16 && (variant == 7 || (variant == 4 && full18_)));
     if (!known) variant = default_variant();
-    // the launches depend on the tiles only through the comparison with their blocks
-    const int nt = tables_.ntiles;
-    const bool divide = (nt < 2 * grid_.low) != (grid_.ntiles < 2 * grid_.low) ||
-                        (nt < 2 * grid_.pk) != (grid_.ntiles < 2 * grid_.pk);
-    if (variant != grid_.variant || mask != grid_.planes_mask || kinds != grid_.kinds || divide) {
+    bool rebuild = false;
+    if (variant != grid_.variant || mask != grid_.planes_mask || kinds != grid_.kinds) {
         grid_ = eng_grid_size(low_, variant, full18_ ? 1 : 0, mask);
-        grid_.ntiles = nt;
         grid_.kinds = kinds;  // the phases the iteration launches (engine.cu)
+        rebuild = true;
+    }
+    const EngGrid before = grid_;
+    if (tables_dirty_ || rebuild) divide_tiles();
+    if (rebuild || !std::equal(grid_.divided, grid_.divided + kEngItemKinds, before.divided)) {
         if (chunk_exec_) {
             HW_CUDA(cudaStreamSynchronize(ctx_->stream));
             cudaGraphExecDestroy(chunk_exec_);

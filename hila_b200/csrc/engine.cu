@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "engine.h"
+#include "engine_parts.h"
 #include "pair.cuh"
 #include "reduce.cuh"
 #include "staggered_math.cuh"
@@ -127,24 +128,22 @@ __device__ __forceinline__ void build_active(const EngPtrs &P, ActiveTable &A) {
     __syncthreads();
 }
 
-// Work items of the hop phases: a tile times a part of its active slots.  With fewer tiles
-// than twice the blocks, a tile's slots are divided (by a power of two) so that the launch has
-// about two items per block; every slot of a tile is still summed over the whole tile, so
-// results do not depend on the division.
+// Work items of the hop phases (engine_parts.h): a tile and one part of its active slots.  Every
+// slot of a tile is summed over the whole tile, so results do not depend on the division.
 struct TileParts {
-    int shift = 0;  // 2^shift items per tile
+    int parts = 1;
+    unsigned magic = 0;  // 2^32 / parts, rounded up
     __device__ TileParts() {}
-    __device__ explicit TileParts(int ntiles) {
-        while ((ntiles << shift) < 2 * (int)gridDim.x && (1 << shift) < kEngMaxRhs) shift++;
-    }
-    __device__ int items(int ntiles) const { return ntiles << shift; }
-    __device__ int tile(int item) const { return item >> shift; }
-    // slots [a0, a1) of na for the item's part, in multiples of `unit` (a power of two); false:
-    // nothing to do (the item still arrives: after the last arrival slots may leave, and the
-    // parts would shift)
+    __device__ explicit TileParts(int n) : parts(n), magic(n > 1 ? 0xffffffffu / n + 1u : 0u) {}
+    __device__ int items(int ntiles) const { return ntiles * parts; }
+    // n / parts, for n < 2^28
+    __device__ int over(int n) const { return parts > 1 ? (int)__umulhi((unsigned)n, magic) : n; }
+    __device__ int tile(int item) const { return over(item); }
+    // slots [a0, a1) of na for the item's part, in multiples of `unit`; false: nothing to do
+    // (the item still arrives: after the last arrival slots may leave, and the parts would shift)
     __device__ bool range(int item, int na, int unit, int &a0, int &a1) const {
-        const int per = (((na + (1 << shift) - 1) >> shift) + unit - 1) & -unit;
-        a0 = (item & ((1 << shift) - 1)) * per;
+        const int per = (over(na + parts - 1) + unit - 1) & -unit;  // part_slots(na, parts, unit)
+        a0 = (item - tile(item) * parts) * per;
         a1 = min(na, a0 + per);
         return a0 < na;
     }
@@ -401,7 +400,7 @@ __device__ __forceinline__ void arrive_and_finish(const EngPtrs &P, const EngLat
 // NR right-hand sides at a time, so links, their third rows and the neighbour
 // indices are shared by the NR solves.  PK (with NR = 2 and FP16 input): the two
 // solves run in the two lanes of packed FP32 instructions (pair.cuh).
-// PARTS: items divide a tile's slots (TileParts).
+// PARTS: items divide a tile's slots (engine_parts.h).
 template <int PHASE, int LOW, int NR, int MINB, bool FULL18, bool PK, bool PARTS>
 __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
     constexpr int SIGN = (PHASE == PH_P1 || PHASE == PH_P2) ? 1 : -1;
@@ -422,13 +421,16 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
     __shared__ int s_tile;
     __shared__ double s_red[NRED > 0 ? kEngMaxRhs : 1][kEngTile / 32];
     const EngTables *T = P.T;
-    const int ntiles = T->ntiles;
     const int max_tiles = T->max_tiles;
-    const bool dyn = T->dyn != 0;
-    const TileParts TP = PARTS ? TileParts(ntiles) : TileParts();
-    const int nitems = PARTS ? TP.items(ntiles) : ntiles;
+    constexpr int KIND = PK ? ITEMS_PK : ITEMS_LOW;
+    const TileParts TP = PARTS ? TileParts(T->parts[KIND]) : TileParts();
+    const int nitems = PARTS ? TP.items(T->ntiles) : T->ntiles;
     // the next item: block + k * grid, or the next value of the phase's counter; the
-    // partial sums are per (slot, tile), so the order does not change any result
+    // partial sums are per (slot, tile), so the order does not change any result.  With an item
+    // per block at most the order is fixed: from the counter the blocks that start first take
+    // them all, and those sit on few SMs (8^4, one FP16 source: 76 us per iteration against 55).
+    // Uneven parts go by the counter: in fixed order a block can meet the larger one each time
+    const bool dyn = (T->dyn != 0 || (PARTS && !T->even[KIND])) && nitems > (int)gridDim.x;
     auto next_item = [&](int cur) {
         if (!dyn) return cur + (int)gridDim.x;
         if (threadIdx.x == 0) s_tile = atomicAdd(P.sched + PHASE, 1);
@@ -864,14 +866,12 @@ void enqueue_rest(const EngPtrs &P, const EngGrid &G, cudaStream_t s, const cuda
     mark(ev, kEngPhases, s);
 }
 
-// One low-precision phase.  A launch with few tiles per block divides their slots (TileParts):
-// FP32, 3 sources at 20x12x28x36 (473 tiles for 888 blocks) P1 51 -> 45, P2 73 -> 64, P4 101 ->
-// 85 us; above two tiles per block the undivided form is as fast or faster (32^4).  (Blocks of
-// three teams on one tile, sharing its staged links and leaving more of the L1: P1 0.36 ->
-// 0.40 ms at 32^4 with 12 sources.)
+// One low-precision phase, its tiles' slots divided where engine_parts.h says so (undivided, the
+// kernel without parts is 1-2% faster).  (Blocks of three teams on one tile, sharing its staged
+// links and leaving more of the L1: P1 0.36 -> 0.40 ms at 32^4 with 12 sources.)
 template <int PHASE, int LOW, int NR, int MINB, bool FULL18, bool PK = false>
 void launch_low(const EngPtrs &P, const EngGrid &G, int blocks, cudaStream_t s) {
-    if (G.ntiles < 2 * blocks)
+    if (G.divided[PK ? ITEMS_PK : ITEMS_LOW])
         k_eng_low<PHASE, LOW, NR, MINB, FULL18, PK, true><<<blocks, kEngTile, 0, s>>>(P);
     else
         k_eng_low<PHASE, LOW, NR, MINB, FULL18, PK, false><<<blocks, kEngTile, 0, s>>>(P);
@@ -1035,7 +1035,7 @@ EngGrid eng_grid_size(int low, int variant, int full18, int planes_mask) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&st, k_stag_low<PH_P1>, kStagLowBlock, 0);
     G.stag = sms * (st < 1 ? 1 : st);
     G.kinds = 1;
-    G.ntiles = 0;
+    for (bool &d : G.divided) d = false;
     G.variant = variant;
     G.full18 = full18;
     G.planes_mask = planes_mask;

@@ -52,6 +52,11 @@ enum EngStatus : int { ENG_RUNNING = 0, ENG_CONVERGED = 1, ENG_MAXITER = 2, ENG_
 enum EngFermion : int { FERM_WILSON = 0, FERM_STAGGERED = 1, FERM_STAGGERED_LOW = 2 };
 enum EngMode : int { ENG_MODE_SOLVE = 0, ENG_MODE_NORMAL = 1 };
 
+// launch grids of the hop phases, each with its own division of the tiles' slots (engine_parts.h):
+// one source per thread, two (packed), the staggered FP16 phases
+enum EngItems : int { ITEMS_LOW = 0, ITEMS_PK = 1, ITEMS_STAG = 2 };
+constexpr int kEngItemKinds = 3;
+
 struct EngLattice {
     Geom g;
     int stride;       // padded sites per parity of every field of this lattice
@@ -117,6 +122,8 @@ struct EngTables {
                  // tiles carry different numbers of active slots); 0: tile = block + k * grid
     EngLattice lat[kEngMaxLat];
     EngProblem prob[kEngMaxProb];
+    int parts[kEngItemKinds];  // parts that a tile's slots are divided into ...
+    int even[kEngItemKinds];   // ... and whether all of them hold as many slots
 };
 
 // device pointers the engine kernels take
@@ -152,7 +159,7 @@ struct EngGrid {
     int full18;   // 1: inner phases read 18-real links (FP32 or FP16); 0: the 12-real links of the precision
     int planes_mask;  // FP64 link formats present: bit 0 = 18 reals, bit 1 = 12 reals
     int stag; // blocks of the staggered FP16 phases
-    int ntiles;  // tiles the launches were shaped for (whether a tile's slots are divided)
+    bool divided[kEngItemKinds];  // whether tiles have more than one part
     int kinds;        // slot kinds whose phases are launched: bit 0 Wilson, bit 1 staggered FP64, bit 2 staggered FP16
 };
 

@@ -92,6 +92,7 @@ class Engine {
     int build_graph();
     void set_ptrs();
     int configure();
+    void divide_tiles();
     int ensure_partials();
 
     hw_context *ctx_;

@@ -220,16 +220,18 @@ __global__ void __launch_bounds__(kStagLowBlock, PHASE == PH_P4 ? 2 : 3) k_stag_
     __shared__ double s_red[NRED > 0 ? kEngMaxRhs : 1][kEngTile / 32];
     const EngTables *T = P.T;
     const int max_tiles = T->max_tiles;
-    const TileParts TP(T->ntiles);
+    const TileParts TP(T->parts[ITEMS_STAG]);
     const int nitems = TP.items(T->ntiles);
     const int team = threadIdx.x / kEngTile, t = threadIdx.x % kEngTile;
     const LinksF16x18Smem<kEngTile> US{s_lx, s_lz, OUTPAR, t};
+    // in fixed order where each block has one item at most (as in k_eng_low)
     auto next_item = [&]() {
+        if (nitems <= (int)gridDim.x) return nitems;
         if (threadIdx.x == 0) s_item = atomicAdd(P.sched + kEngPhases + PHASE, 1);
         __syncthreads();
         return s_item;
     };
-    for (int item = next_item(); item < nitems; item = next_item()) {
+    for (int item = nitems <= (int)gridDim.x ? (int)blockIdx.x : next_item(); item < nitems; item = next_item()) {
         const int tile = TP.tile(item);
         const int l = find_lattice(T, tile);
         const EngLattice &La = T->lat[l];

@@ -38,6 +38,28 @@ def test_divided_tiles(hw, ctx, dims, counts, precision):
             assert batch[k] == alone[k], (n, k)
 
 
+@pytest.mark.parametrize("precision", ["f16", "f32"])
+def test_divided_lattices(hw, ctx, precision):
+    """Lattices with 1, 3 and 13 solves in one launch, divided by one rule (their solves leave at
+    different iterations): the bits of the solves alone."""
+    delta = 0.005 if precision == "f16" else 1e-5
+    reqs, alone = [], []
+    for dims, n, kappa in (((8, 8, 8, 12), 13, 0.12), ((2, 4, 6, 2), 1, 0.1), ((12, 12, 12, 12), 3, 0.11)):
+        lat = hw.Lattice(ctx, dims)
+        D = hw.Dirac_Wilson_evenodd(kappa, hw.GaugeField(lat, hw.generate_links(dims, 0.3, 3), 18 if n == 3 else 12))
+        for k in range(n):
+            tol = TOL * 10 ** (k % 4)
+            reqs.append((D, hw.Field(lat, hw.generate_spinor(dims, 50 + k, hw.EVEN)), hw.Field(lat), tol))
+    for D, b, x, tol in reqs:
+        r = hw.batch_solve(ctx, [(D, b, x, tol)], precision=precision, delta=delta)[0]
+        assert r.converged
+        alone.append((r.iterations, x.download().tobytes()))
+        x.zero()
+    res = hw.batch_solve(ctx, reqs, precision=precision, delta=delta)
+    for r, (_, _, x, _), a in zip(res, reqs, alone):
+        assert (r.iterations, x.download().tobytes()) == a
+
+
 @pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 4, 2, 6), (8, 8, 8, 8), (12, 12, 12, 14)])
 @pytest.mark.parametrize("normal", [False, True])
 def test_staggered_pairs(hw, ctx, dims, normal):

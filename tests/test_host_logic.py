@@ -1,5 +1,6 @@
 """Host-side logic that needs no GPU, compiled and run on the CPU: the sizes of the grid
-reductions (hila_b200/csrc/hop_shapes.h) by tests/cpp/test_reductions.cpp."""
+reductions (hila_b200/csrc/hop_shapes.h) by tests/cpp/test_reductions.cpp, the division of the
+engine's tiles (engine_parts.h) by test_parts.cpp."""
 import os
 import subprocess
 
@@ -21,3 +22,7 @@ def compile_and_run(tmp_path, name, *flags):
 
 def test_reduction_sizes(tmp_path):
     assert "reduction sizes passed" in compile_and_run(tmp_path, "test_reductions")
+
+
+def test_parts(tmp_path):
+    assert "parts passed" in compile_and_run(tmp_path, "test_parts")

@@ -417,55 +417,47 @@ void Engine::set_ptrs() {
 int Engine::build_graph() {
     set_ptrs();
     cudaStream_t s = ctx_->stream;
-    cudaGraph_t g = nullptr;
-    HW_CUDA(cudaGraphCreate(&g, 0));
+    int rc;
+    GraphHolder G;
+    HW_CUDA(cudaGraphCreate(&G.g, 0));
     cudaGraphConditionalHandle cond;
-    HW_CUDA(cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault));
+    HW_CUDA(cudaGraphConditionalHandleCreate(&cond, G.g, 1, cudaGraphCondAssignDefault));
     // chunk begin
-    HW_CUDA(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    eng_enqueue_chunk_begin(ptrs_, s);
-    cudaGraph_t tmp = nullptr;
-    HW_CUDA(cudaStreamEndCapture(s, &tmp));
+    if ((rc = capture_into(s, G.g, nullptr, 0, [&] { return eng_enqueue_chunk_begin(ptrs_, s), HW_OK; })) != HW_OK)
+        return rc;
     size_t n = 0;
-    HW_CUDA(cudaGraphGetNodes(g, nullptr, &n));
+    HW_CUDA(cudaGraphGetNodes(G.g, nullptr, &n));
     std::vector<cudaGraphNode_t> nodes(n);
-    HW_CUDA(cudaGraphGetNodes(g, nodes.data(), &n));
-    cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
-    np.conditional.handle = cond;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t wnode;
-    HW_CUDA(cudaGraphAddNode(&wnode, g, nodes.data(), nodes.size(), &np));
-    cudaGraph_t body = np.conditional.phGraph_out[0];
+    HW_CUDA(cudaGraphGetNodes(G.g, nodes.data(), &n));
+    cudaGraphNode_t loop;
+    cudaGraph_t body, update = nullptr;
+    if ((rc = add_conditional(G.g, nodes.data(), n, cond, cudaGraphCondTypeWhile, &loop, &body)) != HW_OK) return rc;
     // body: inner phases -> gate -> IF (a reliable update is pending) { R1..R5L } -> P5 -> control.
     // The seven (with staggered slots fourteen) phases of an update are not launched in the
     // other iterations, where each returned at once after some 2 us.
     cudaGraphConditionalHandle ru;
     HW_CUDA(cudaGraphConditionalHandleCreate(&ru, body, 0, 0));
-    cudaGraphNodeParams ip = {cudaGraphNodeTypeConditional};
-    ip.conditional.handle = ru;
-    ip.conditional.type = cudaGraphCondTypeIf;
-    ip.conditional.size = 1;
-    HW_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_INNER);
-    eng_enqueue_gate(ptrs_, ru, s);
-    cudaStreamCaptureStatus status;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t ndeps = 0;
-    HW_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &ndeps));
-    cudaGraphNode_t inode;
-    HW_CUDA(cudaGraphAddNode(&inode, body, deps, ndeps, &ip));
-    HW_CUDA(cudaStreamUpdateCaptureDependencies(s, &inode, 1, cudaStreamSetCaptureDependencies));
-    eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_P5);
-    eng_enqueue_control(ptrs_, kEngMaxProb, 0, cond, 1, s);
-    HW_CUDA(cudaStreamEndCapture(s, &tmp));
-    HW_CUDA(cudaStreamBeginCaptureToGraph(s, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal));
-    eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_RU);
-    HW_CUDA(cudaStreamEndCapture(s, &tmp));
-    cudaError_t e = cudaGraphInstantiate(&chunk_exec_, g, 0);
-    cudaGraphDestroy(g);
-    HW_CUDA(e);
+    rc = capture_into(s, body, nullptr, 0, [&]() -> int {
+        eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_INNER);
+        eng_enqueue_gate(ptrs_, ru, s);
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t *deps = nullptr;
+        size_t ndeps = 0;
+        HW_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &ndeps));
+        cudaGraphNode_t node;
+        const int e = add_conditional(body, deps, ndeps, ru, cudaGraphCondTypeIf, &node, &update);
+        if (e != HW_OK) return e;
+        HW_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
+        eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_P5);
+        eng_enqueue_control(ptrs_, kEngMaxProb, 0, cond, 1, s);
+        return HW_OK;
+    });
+    if (rc != HW_OK) return rc;
+    rc = capture_into(s, update, nullptr, 0, [&] {
+        return eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_RU), HW_OK;
+    });
+    if (rc != HW_OK) return rc;
+    HW_CUDA(cudaGraphInstantiate(&chunk_exec_, G.g, 0));
     return HW_OK;
 }
 

@@ -10,34 +10,13 @@
 #include <string>
 #include <vector>
 
-#include "../../include/hila_b200.h"
+#include "errors.h"
+#include "graph_build.h"
 #include "kernels.h"
 
 namespace hw {
 
 class Engine;
-
-// ------------------------------------------------------------------ errors
-
-void set_error(const char *fmt, ...);
-void clear_error();
-
-#define HW_CHECK_ARG(cond, ...)              \
-    do {                                     \
-        if (!(cond)) {                       \
-            ::hw::set_error(__VA_ARGS__);    \
-            return HW_ERR_INVALID;           \
-        }                                    \
-    } while (0)
-
-#define HW_CUDA(call)                                                                              \
-    do {                                                                                           \
-        cudaError_t e_ = (call);                                                                   \
-        if (e_ != cudaSuccess) {                                                                   \
-            ::hw::set_error("%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
-            return e_ == cudaErrorMemoryAllocation ? HW_ERR_OOM : HW_ERR_CUDA;                     \
-        }                                                                                          \
-    } while (0)
 
 // RAII device buffer
 struct DevBuf {
@@ -113,8 +92,8 @@ struct CgWorkspace {
         double kappa = 0, acc2 = 0, diag = 1;
         int maxiter = 0, mode = 0, planes = 0;
         bool operator==(const Key &o) const {
-            return links == o.links && planes == o.planes && red == o.red && in == o.in && out == o.out && kappa == o.kappa && acc2 == o.acc2 &&
-                   diag == o.diag && maxiter == o.maxiter && mode == o.mode;
+            return links == o.links && planes == o.planes && red == o.red && in == o.in && out == o.out &&
+                   kappa == o.kappa && acc2 == o.acc2 && diag == o.diag && maxiter == o.maxiter && mode == o.mode;
         }
     } key;
     bool allocated = false;
@@ -177,10 +156,6 @@ struct hw_stag_field {
 namespace hw {
 int ensure_workspace(hw_lattice *lat);
 int ensure_reduction_capacity(hw_context *ctx, long nblocks);
-// Loop graph of a CG: WHILE(status == running) { body }, where body enqueues one iteration on
-// the stream and its last kernel sets the handle it is given (loop_next); replaces *exec
-template <class Body>
-int build_loop_graph(cudaStream_t s, cudaGraphExec_t *exec, Body body);
 int ensure_stage(hw_context *ctx, size_t bytes);
 // pick the fastest FP64 hop launch shape for this lattice once (HW_HOP_VARIANT overrides)
 int tune_hop(hw_lattice *lat, const hw_gauge *G);
@@ -199,29 +174,4 @@ inline int force_buffer(hw_context *ctx, size_t bytes, DevBuf &own, void **out) 
 // caller holds the context's lock.
 int copy_to_host(hw_context *ctx, void *dst, const void *src, size_t bytes);
 void destroy_engines(hw_context *ctx);
-
-template <class Body>
-int build_loop_graph(cudaStream_t s, cudaGraphExec_t *exec, Body body) {
-    if (*exec) cudaGraphExecDestroy(*exec);
-    *exec = nullptr;
-    cudaGraph_t g = nullptr;
-    HW_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle cond;
-    HW_CUDA(cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
-    np.conditional.handle = cond;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t wnode;
-    HW_CUDA(cudaGraphAddNode(&wnode, g, nullptr, 0, &np));
-    HW_CUDA(cudaStreamBeginCaptureToGraph(s, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal));
-    body(cond);
-    cudaGraph_t captured = nullptr;
-    HW_CUDA(cudaStreamEndCapture(s, &captured));
-    const cudaError_t e = cudaGraphInstantiate(exec, g, 0);
-    cudaGraphDestroy(g);
-    HW_CUDA(e);
-    return HW_OK;
-}
 }  // namespace hw

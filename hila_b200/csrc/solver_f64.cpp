@@ -87,40 +87,14 @@ struct F64Solve {
 };
 
 int build_graphs(F64Solve &S, double acc2, int maxiter, cudaGraphExec_t *init_exec, cudaGraphExec_t *loop_exec) {
-    cudaStream_t s = S.s;
-    // init graph
-    cudaGraph_t gi = nullptr;
-    HW_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    S.enqueue_init(acc2, maxiter);
-    HW_CUDA(cudaStreamEndCapture(s, &gi));
-    cudaError_t e = cudaGraphInstantiate(init_exec, gi, 0);
-    cudaGraphDestroy(gi);
-    HW_CUDA(e);
-
-    // loop graph: WHILE(status == running) { body } -> residual check
-    cudaGraph_t g = nullptr;
-    HW_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle cond;
-    HW_CUDA(cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
-    np.conditional.handle = cond;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t wnode;
-    HW_CUDA(cudaGraphAddNode(&wnode, g, nullptr, 0, &np));
-    cudaGraph_t body = np.conditional.phGraph_out[0];
-    HW_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    S.enqueue_body(cond, 1);
-    cudaGraph_t body_out = nullptr;
-    HW_CUDA(cudaStreamEndCapture(s, &body_out));
-    HW_CUDA(cudaStreamBeginCaptureToGraph(s, g, &wnode, nullptr, 1, cudaStreamCaptureModeThreadLocal));
-    S.enqueue_check();
-    cudaGraph_t g_out = nullptr;
-    HW_CUDA(cudaStreamEndCapture(s, &g_out));
-    e = cudaGraphInstantiate(loop_exec, g, 0);
-    cudaGraphDestroy(g);
-    HW_CUDA(e);
-    return HW_OK;
+    int rc;
+    GraphHolder init;
+    HW_CUDA(cudaGraphCreate(&init.g, 0));
+    rc = capture_into(S.s, init.g, nullptr, 0, [&] { return S.enqueue_init(acc2, maxiter), HW_OK; });
+    if (rc != HW_OK) return rc;
+    HW_CUDA(cudaGraphInstantiate(init_exec, init.g, 0));
+    return build_loop_graph(
+        S.s, loop_exec, [&](cudaGraphConditionalHandle cond) { S.enqueue_body(cond, 1); }, [&] { S.enqueue_check(); });
 }
 
 int read_state(hw_context *ctx) {
@@ -210,7 +184,7 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
             S.enqueue_check();
         }
         if ((rc = read_state(ctx)) != HW_OK) return rc;
-            true_res = h->res_den2 > 0 ? std::sqrt(h->res_num2 / h->res_den2) : 0.0;
+        true_res = h->res_den2 > 0 ? std::sqrt(h->res_num2 / h->res_den2) : 0.0;
     }
     HW_CUDA(cudaEventRecord(ctx->ev1, S.s));
     HW_CUDA(cudaEventSynchronize(ctx->ev1));

@@ -1,11 +1,13 @@
 """Host-side logic that needs no GPU, compiled and run on the CPU: the sizes of the grid
 reductions (hila_b200/csrc/hop_shapes.h) by tests/cpp/test_reductions.cpp, the division of the
-engine's tiles (engine_parts.h) by test_parts.cpp."""
+engine's tiles (engine_parts.h) by test_parts.cpp, graph construction (graph_build.h) over a
+fake CUDA runtime by test_graph_build.cpp."""
 import os
 import subprocess
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "hila_b200", "csrc")
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
 
 
 def compile_and_run(tmp_path, name, *flags):
@@ -26,3 +28,7 @@ def test_reduction_sizes(tmp_path):
 
 def test_parts(tmp_path):
     assert "parts passed" in compile_and_run(tmp_path, "test_parts")
+
+
+def test_graph_build(tmp_path):
+    assert "graph construction passed" in compile_and_run(tmp_path, "test_graph_build", "-I", CUDA_INCLUDE)

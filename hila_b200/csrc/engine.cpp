@@ -53,7 +53,7 @@ Engine::~Engine() {
         cudaSetDevice(ctx_->device);
         cudaStreamSynchronize(ctx_->stream);
     }
-    if (chunk_exec_) cudaGraphExecDestroy(chunk_exec_);
+    graphs_.clear();
     if (pinned_states_) cudaFreeHost(pinned_states_);
     if (pinned_ctl_) cudaFreeHost(pinned_ctl_);
     if (pinned_work_) cudaFreeHost(pinned_work_);
@@ -112,10 +112,8 @@ int Engine::ensure_partials() {
     int rc = d_partials_.alloc(sizeof(double) * 2 * kEngMaxProb * cap);
     if (rc != HW_OK) return rc;
     partial_tiles_ = cap;
-    if (chunk_exec_) {  // pointer changed: rebuild the graph
-        cudaGraphExecDestroy(chunk_exec_);
-        chunk_exec_ = nullptr;
-    }
+    graphs_.clear();  // they hold the old pointer
+    chunk_exec_ = nullptr;
     return HW_OK;
 }
 
@@ -414,7 +412,21 @@ void Engine::set_ptrs() {
     ptrs_.sched = d_sched_.as<int>();
 }
 
-int Engine::build_graph() {
+// chunk_exec_ for the launches of grid_
+int Engine::chunk_graph() {
+    unsigned key = (unsigned)grid_.variant | (unsigned)grid_.planes_mask << 8 | (unsigned)grid_.kinds << 10;
+    for (int k = 0; k < kEngItemKinds; k++) key |= (unsigned)grid_.divided[k] << (13 + k);
+    if ((chunk_exec_ = graphs_.find(key)) != nullptr) return HW_OK;
+    if (graphs_.full()) HW_CUDA(cudaStreamSynchronize(ctx_->stream));
+    cudaGraphExec_t exec = nullptr;
+    const int rc = build_graph(&exec);
+    if (rc != HW_OK) return rc;
+    graphs_.put(key, exec);
+    chunk_exec_ = exec;
+    return HW_OK;
+}
+
+int Engine::build_graph(cudaGraphExec_t *exec) {
     set_ptrs();
     cudaStream_t s = ctx_->stream;
     int rc;
@@ -457,7 +469,7 @@ int Engine::build_graph() {
         return eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_RU), HW_OK;
     });
     if (rc != HW_OK) return rc;
-    HW_CUDA(cudaGraphInstantiate(&chunk_exec_, G.g, 0));
+    HW_CUDA(cudaGraphInstantiate(exec, G.g, 0));
     return HW_OK;
 }
 
@@ -486,13 +498,6 @@ int Engine::configure() {
     for (int j = 0; j < kEngMaxProb; j++)
         if (slots_[j].used) kinds |= 1 << host_states_[j].fermion;
     if (mask == 0) mask = 1;
-    // a kind that was there keeps its phases for some chunks after its last slot has gone, so
-    // that a stream that alternates does not rebuild the graph each time
-    for (int k = 0; k < 3; k++) {
-        kind_idle_[k] = (kinds >> k & 1) ? 0 : kind_idle_[k] + 1;
-        if ((grid_.kinds >> k & 1) && kinds && kind_idle_[k] <= kKindIdleChunks && kind_seen_[k]) kinds |= 1 << k;
-        if (kinds >> k & 1) kind_seen_[k] = true;
-    }
     if (kinds == 0) kinds = grid_.kinds;
     int variant = want_variant_ ? want_variant_ : default_variant();
     if (const char *env = std::getenv("HW_ENGINE_VARIANT")) variant = std::atoi(env);
@@ -501,21 +506,14 @@ int Engine::configure() {
     const bool known =
         variant == 2 || (low_ == LOW_F16 && (variant == 7 || (variant == 4 && full18_)));
     if (!known) variant = default_variant();
-    bool rebuild = false;
-    if (variant != grid_.variant || mask != grid_.planes_mask || kinds != grid_.kinds) {
+    const EngGrid before = grid_;
+    const bool other = variant != grid_.variant || mask != grid_.planes_mask || kinds != grid_.kinds;
+    if (other) {
         grid_ = eng_grid_size(low_, variant, full18_ ? 1 : 0, mask);
         grid_.kinds = kinds;  // the phases the iteration launches (engine.cu)
-        rebuild = true;
     }
-    const EngGrid before = grid_;
-    if (tables_dirty_ || rebuild) divide_tiles();
-    if (rebuild || !std::equal(grid_.divided, grid_.divided + kEngItemKinds, before.divided)) {
-        if (chunk_exec_) {
-            HW_CUDA(cudaStreamSynchronize(ctx_->stream));
-            cudaGraphExecDestroy(chunk_exec_);
-            chunk_exec_ = nullptr;
-        }
-    }
+    if (tables_dirty_ || other) divide_tiles();
+    if (other || !std::equal(grid_.divided, grid_.divided + kEngItemKinds, before.divided)) chunk_exec_ = nullptr;
     return HW_OK;
 }
 
@@ -571,7 +569,7 @@ int Engine::launch_chunk(int iters) {
         tune_pending_.shape = shape;
         return launch_chunk_timed(iters);
     }
-    if (use_graph_ && !chunk_exec_ && (rc = build_graph()) != HW_OK) return rc;
+    if (use_graph_ && !chunk_exec_ && (rc = chunk_graph()) != HW_OK) return rc;
     if ((rc = upload_tables()) != HW_OK) return rc;
     if (ctx_->engine_profile) return launch_chunk_profiled(iters);
     if (!use_graph_) {

@@ -7,6 +7,7 @@
 
 #include "engine.h"
 #include "engine_tune.h"
+#include "graph_cache.h"
 #include "hw_internal.h"
 
 namespace hw {
@@ -89,7 +90,8 @@ class Engine {
 
   private:
     int ensure_slot_buffers(int slot, int stride);
-    int build_graph();
+    int chunk_graph();
+    int build_graph(cudaGraphExec_t *exec);
     void set_ptrs();
     int configure();
     void divide_tiles();
@@ -127,9 +129,6 @@ class Engine {
     int launch_chunk_profiled(int iters);
     int launch_chunk_timed(int iters);
     void tune_collect();
-    static constexpr int kKindIdleChunks = 16;
-    int kind_idle_[3] = {0, 0, 0};  // chunks since a slot of the kind was last in use (configure)
-    bool kind_seen_[3] = {false, false, false};
     int want_variant_ = 0;  // the tuner's shape for the next chunks (0: the default)
     std::map<int, TuneEntry> tune_;
     std::vector<cudaEvent_t> tune_ev_;  // kTuneMaxIters x (kEngPhases + 1)
@@ -140,7 +139,11 @@ class Engine {
     size_t partial_tiles_ = 0;
     EngGrid grid_{};
     EngPtrs ptrs_{};
-    cudaGraphExec_t chunk_exec_ = nullptr;
+    static void destroy_exec(cudaGraphExec_t x) { cudaGraphExecDestroy(x); }
+    // chunk graphs by launch shape, link formats, slot kinds and divided phases (a build and the
+    // end of the graph before took 0.5 ms, and a stream of unlike lattices goes back and forth)
+    GraphCache<cudaGraphExec_t, 16, destroy_exec> graphs_;
+    cudaGraphExec_t chunk_exec_ = nullptr;  // the one of grid_, once made (owned by graphs_)
     bool tables_dirty_ = true;
     bool use_graph_ = true;
     bool full18_ = false;

@@ -1,7 +1,8 @@
 """Host-side logic that needs no GPU, compiled and run on the CPU: the sizes of the grid
 reductions (hila_b200/csrc/hop_shapes.h) by tests/cpp/test_reductions.cpp, the division of the
 engine's tiles (engine_parts.h) by test_parts.cpp, graph construction (graph_build.h) over a
-fake CUDA runtime by test_graph_build.cpp."""
+fake CUDA runtime by test_graph_build.cpp, the cache of graphs (graph_cache.h) by
+test_graph_cache.cpp."""
 import os
 import subprocess
 
@@ -32,3 +33,7 @@ def test_parts(tmp_path):
 
 def test_graph_build(tmp_path):
     assert "graph construction passed" in compile_and_run(tmp_path, "test_graph_build", "-I", CUDA_INCLUDE)
+
+
+def test_graph_cache(tmp_path):
+    assert "graph cache passed" in compile_and_run(tmp_path, "test_graph_cache")

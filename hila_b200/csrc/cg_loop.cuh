@@ -26,6 +26,7 @@ __device__ __forceinline__ void cg_start(CgState *st, double rr, double bb, doub
     st->maxiter = maxiter;
     st->alpha = st->beta = 0.0;
     st->do_pupdate = 0;
+    st->bodies = 0;
     if (!isfinite(rr) || !isfinite(bb))
         st->status = CG_BREAKDOWN;
     else if (bb == 0.0)

@@ -486,6 +486,7 @@ struct FinCgInit {
         st->maxiter = maxiter;
         st->alpha = st->beta = 0.0;
         st->do_pupdate = 0;
+        st->bodies = 0;
         if (!isfinite(tot[0]) || !isfinite(tot[1]))
             st->status = CG_BREAKDOWN;
         else if (tot[1] == 0.0 || tot[0] < st->target_rr)
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(kVecBlock) k_cg_init(int Vh, SpinorF64 src, Sp
 }
 
 // Last kernel of every CG loop-body iteration
-__global__ void __launch_bounds__(kVecBlock) k_cg_pupdate(int Vh, SpinorF64 r, SpinorF64 p, const CgState *st,
+__global__ void __launch_bounds__(kVecBlock) k_cg_pupdate(int Vh, SpinorF64 r, SpinorF64 p, CgState *st,
                                                           cudaGraphConditionalHandle cond, int use_cond) {
     if (blockIdx.x == 0 && threadIdx.x == 0) loop_next(st, cond, use_cond);
     if (!st->do_pupdate) return;

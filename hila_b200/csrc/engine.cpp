@@ -350,6 +350,7 @@ int Engine::admit(int lat, double kappa, double2 *b, double2 *x, double tol, int
     P.t64 = B.t64.as<double2>();
     L.prob[L.nprob++] = slot;
     slots_[slot].used = true;
+    slots_[slot].launches0 = launches_total_;
     slots_[slot].lat = lat;
     tables_dirty_ = true;
 
@@ -461,7 +462,7 @@ int Engine::build_graph(cudaGraphExec_t *exec) {
         if (e != HW_OK) return e;
         HW_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
         eng_enqueue_iteration(low_, ptrs_, grid_, s, nullptr, ENG_PART_P5);
-        eng_enqueue_control(ptrs_, kEngMaxProb, 0, cond, 1, s);
+        eng_enqueue_control(ptrs_, grid_, kEngMaxProb, 0, cond, 1, s);
         return HW_OK;
     });
     if (rc != HW_OK) return rc;
@@ -577,7 +578,7 @@ int Engine::launch_chunk(int iters) {
         eng_enqueue_chunk_begin(ptrs_, ctx_->stream);
         for (int k = 0; k < iters; k++) {
             eng_enqueue_iteration(low_, ptrs_, grid_, ctx_->stream);
-            eng_enqueue_control(ptrs_, kEngMaxProb, iters, 0, 0, ctx_->stream);
+            eng_enqueue_control(ptrs_, grid_, kEngMaxProb, iters, 0, 0, ctx_->stream);
         }
         HW_CUDA(cudaGetLastError());
         return HW_OK;
@@ -604,7 +605,7 @@ int Engine::launch_chunk_timed(int iters) {
     for (int k = 0; k < iters; k++) {
         const cudaEvent_t *ev = k < tune_pending_.iters ? &tune_ev_[(size_t)k * (kEngPhases + 1)] : nullptr;
         eng_enqueue_iteration(low_, ptrs_, grid_, ctx_->stream, ev);
-        eng_enqueue_control(ptrs_, kEngMaxProb, iters, 0, 0, ctx_->stream);
+        eng_enqueue_control(ptrs_, grid_, kEngMaxProb, iters, 0, 0, ctx_->stream);
     }
     HW_CUDA(cudaGetLastError());
     return HW_OK;
@@ -660,7 +661,7 @@ int Engine::launch_chunk_profiled(int iters) {
         if (running == 0) break;
         std::memcpy(work_seen_, pinned_work_, sizeof(work_seen_));
         eng_enqueue_iteration(low_, ptrs_, grid_, ctx_->stream, prof_ev_);
-        eng_enqueue_control(ptrs_, kEngMaxProb, iters, 0, 0, ctx_->stream);
+        eng_enqueue_control(ptrs_, grid_, kEngMaxProb, iters, 0, 0, ctx_->stream);
         int rc;
         if ((rc = read_states()) != HW_OK) return rc;
         for (int ph = 0; ph < kEngPhases; ph++) {
@@ -707,7 +708,7 @@ int Engine::read_states() {
     HW_CUDA(cudaMemcpyAsync(pinned_work_, d_work_.ptr, d_work_.bytes, cudaMemcpyDeviceToHost, ctx_->stream));
     HW_CUDA(cudaStreamSynchronize(ctx_->stream));
     HW_CUDA(cudaGetLastError());
-    bodies_total_ = reinterpret_cast<const unsigned long long *>(pinned_ctl_ + 6)[0];
+    launches_total_ = reinterpret_cast<const unsigned long long *>(pinned_ctl_ + 6)[0];
     for (int j = 0; j < kEngMaxProb; j++)
         if (slots_[j].used) host_states_[j] = pinned_states_[j];
     tune_collect();

@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(kEngTile) k_eng_vec(EngPtrs P) {
 // running slots, and keeps the chunk's WHILE loop going while some slot runs
 // and fewer than `chunk` iterations ran.  No waiting: the loop is bounded by
 // `chunk` and by every slot's maxiter.
-__global__ void k_eng_control(EngPtrs P, int nprob, int chunk, cudaGraphConditionalHandle h, int use_cond) {
+__global__ void k_eng_control(EngPtrs P, int nprob, int chunk, int kernels, int ru_kernels, cudaGraphConditionalHandle h, int use_cond) {
     __shared__ int running;
     if (threadIdx.x == 0) running = 0;
     __syncthreads();
@@ -745,8 +745,8 @@ __global__ void k_eng_control(EngPtrs P, int nprob, int chunk, cudaGraphConditio
         const int it = P.ctl[0] + 1;
         P.ctl[0] = it;
         P.ctl[1] = running;
+        reinterpret_cast<unsigned long long *>(P.ctl + 6)[0] += kernels + (P.ctl[2] ? ru_kernels : 0);
         P.ctl[2] = 0;  // pending reliable updates were served this iteration
-        reinterpret_cast<unsigned long long *>(P.ctl + 6)[0] += 1;  // loop bodies since init
         if (use_cond) cudaGraphSetConditional(h, (running > 0 && it < chunk) ? 1u : 0u);
     }
 }
@@ -756,6 +756,7 @@ __global__ void k_eng_gate(EngPtrs P, cudaGraphConditionalHandle h) { cudaGraphS
 
 __global__ void k_eng_chunk_begin(EngPtrs P) {
     P.ctl[0] = 0;
+    reinterpret_cast<unsigned long long *>(P.ctl + 6)[0] += 1;  // this kernel
     for (int k = 0; k < 2 * kEngPhases; k++) P.sched[k] = 0;
 }
 
@@ -987,9 +988,30 @@ void eng_enqueue_iteration(int low, const EngPtrs &P, const EngGrid &G, cudaStre
 
 void eng_enqueue_gate(const EngPtrs &P, cudaGraphConditionalHandle h, cudaStream_t s) { k_eng_gate<<<1, 1, 0, s>>>(P, h); }
 
-void eng_enqueue_control(const EngPtrs &P, int nprob, int chunk, cudaGraphConditionalHandle h, int use_cond,
-                         cudaStream_t s) {
-    k_eng_control<<<1, 64, 0, s>>>(P, nprob, chunk, h, use_cond);
+// kernels that eng_enqueue_iteration launches for these parts
+static int iteration_kernels(const EngGrid &G, int parts) {
+    int n = 0;
+    if (G.kinds & 1) {
+        const int formats = (G.planes_mask & 1) + (G.planes_mask >> 1 & 1);
+        if (parts & ENG_PART_INNER) n += 4;
+        if (parts & ENG_PART_RU) n += 3 + 4 * formats;  // R1, R4L, R5L; R2, R3, R4, R5 per link format
+        if (parts & ENG_PART_P5) n += 1;
+    }
+    const int stag = (G.kinds >> 1 & 1) + (G.kinds >> 2 & 1);
+    if (parts & ENG_PART_INNER) n += 4 * stag;
+    if (stag && (parts & ENG_PART_RU)) n += 7;
+    if (parts & ENG_PART_P5) n += stag;
+    return n;
+}
+
+void eng_enqueue_control(const EngPtrs &P, const EngGrid &G, int nprob, int chunk, cudaGraphConditionalHandle h,
+                         int use_cond, cudaStream_t s) {
+    // a graph's body: the gate and this kernel too, and the update's kernels where it ran; a host
+    // loop launches every part each time, and no gate
+    const int kernels = use_cond ? iteration_kernels(G, ENG_PART_INNER | ENG_PART_P5) + 2
+                                 : iteration_kernels(G, ENG_PART_ALL) + 1;
+    const int ru_kernels = use_cond ? iteration_kernels(G, ENG_PART_RU) : 0;
+    k_eng_control<<<1, 64, 0, s>>>(P, nprob, chunk, kernels, ru_kernels, h, use_cond);
 }
 
 void eng_enqueue_chunk_begin(const EngPtrs &P, cudaStream_t s) { k_eng_chunk_begin<<<1, 1, 0, s>>>(P); }

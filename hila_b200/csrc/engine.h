@@ -134,7 +134,8 @@ struct EngPtrs {
     unsigned *tickets;    // one per lattice
     int *ctl;             // [0] iterations run in this chunk, [1] running slots,
                           // [2] reliable updates requested in this iteration,
-                          // [3] iteration limit of a chunk (control kernel with chunk <= 0)
+                          // [3] iteration limit of a chunk (control kernel with chunk <= 0),
+                          // [6..7] kernels run since init (64 bits)
     unsigned long long *work;  // kEngPhases x kEngWorkKinds cumulative work units (below)
     int *sched;           // item counters of the inner phases' dynamic order: kEngPhases of the Wilson
                           // phases, then kEngPhases of the staggered FP16 ones (zeroed at the start
@@ -184,8 +185,9 @@ void eng_enqueue_iteration(int low, const EngPtrs &P, const EngGrid &G, cudaStre
 // Sets the handle of a graph's IF node by whether some slot asked for a reliable update.
 void eng_enqueue_gate(const EngPtrs &P, cudaGraphConditionalHandle h, cudaStream_t s);
 // While-loop control: counts running slots, stops after `chunk` iterations or when none runs.
-void eng_enqueue_control(const EngPtrs &P, int nprob, int chunk, cudaGraphConditionalHandle h, int use_cond,
-                         cudaStream_t s);
+// Counts the kernels of the iteration (G: the grid its phases were launched with).
+void eng_enqueue_control(const EngPtrs &P, const EngGrid &G, int nprob, int chunk, cudaGraphConditionalHandle h,
+                         int use_cond, cudaStream_t s);
 void eng_enqueue_chunk_begin(const EngPtrs &P, cudaStream_t s);
 // Convert FP64 link planes to the 12-real FP32 / FP16 planes of the inner solve.
 void eng_convert_links(const Geom &g, const double2 *l64, int planes, int stride, float4 *l32, uint4 *l16a,

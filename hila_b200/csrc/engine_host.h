@@ -23,6 +23,7 @@ struct SlotBuffers {
 struct SlotInfo {
     bool used = false;
     int lat = -1;
+    unsigned long long launches0 = 0;  // the engine's kernels when the slot was admitted
 };
 
 // Online choice of the inner phases' launch shape: the candidates (engine_tune.h) are
@@ -59,8 +60,9 @@ class Engine {
     int launch_chunk(int iters);
     // copy the slot states to the host mirror (synchronises the stream)
     int read_states();
-    // loop bodies (10 phase kernels + 1 control kernel each) run since init, as of the last read_states
-    unsigned long long bodies_total() const { return bodies_total_; }
+    // kernels run since init, and since a slot was admitted, as of the last read_states
+    unsigned long long launches_total() const { return launches_total_; }
+    unsigned long long launches_of(int slot) const { return launches_total_ - slots_[slot].launches0; }
     // per-phase device time and work units (engine.h, kEngWorkKinds) of the launches
     // that did work, while the context's engine profiling is on (iterations then run
     // from a synchronising host loop)
@@ -122,7 +124,7 @@ class Engine {
     unsigned long long *pinned_work_ = nullptr;  // kEngPhases x kEngWorkKinds, as of the last read_states
     unsigned long long work_seen_[kEngPhases * kEngWorkKinds] = {};
     unsigned long long prof_work_[kEngPhases * kEngWorkKinds] = {};
-    unsigned long long bodies_total_ = 0;
+    unsigned long long launches_total_ = 0;
     cudaEvent_t prof_ev_[kEngPhases + 1] = {};
     long prof_n_[kEngPhases] = {};
     double prof_ms_[kEngPhases] = {};

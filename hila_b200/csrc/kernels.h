@@ -62,6 +62,7 @@ struct CgState {
     int iter, maxiter;
     int status;        // CG_RUNNING / CG_CONVERGED / CG_MAXITER / CG_BREAKDOWN
     int do_pupdate;    // whether the iteration's last kernel forms p (its CG update ran)
+    int bodies;        // loop bodies run
 };
 enum : int { CG_RUNNING = 0, CG_CONVERGED = 1, CG_MAXITER = 2, CG_BREAKDOWN = 3 };
 
@@ -69,7 +70,8 @@ enum : int { CG_RUNNING = 0, CG_CONVERGED = 1, CG_MAXITER = 2, CG_BREAKDOWN = 3 
 // Keeps a graph's while loop going while the solve runs: called by one thread of an iteration's
 // last kernel (the kernel always runs, so the loop ends even when the others returned early;
 // the iteration counter is bounded by maxiter, so the loop is bounded).
-__device__ __forceinline__ void loop_next(const CgState *st, cudaGraphConditionalHandle cond, int use_cond) {
+__device__ __forceinline__ void loop_next(CgState *st, cudaGraphConditionalHandle cond, int use_cond) {
+    st->bodies += 1;
     if (use_cond) cudaGraphSetConditional(cond, st->status == CG_RUNNING ? 1u : 0u);
 }
 #endif

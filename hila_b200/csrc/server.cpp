@@ -572,10 +572,8 @@ void server_loop(hw_server *S) {
                 lk.unlock();
                 rc = S->eng->read_states();
                 lk.lock();
-                // every chunk graph runs one begin kernel, then 7 kernels per loop body (the seven
-                // more of a body with a reliable update are not counted)
                 S->stats.chunks++;
-                S->stats.kernel_launches = S->layout_launches + S->stats.chunks + 7 * S->eng->bodies_total();
+                S->stats.kernel_launches = S->layout_launches + S->eng->launches_total();
             }
             S->stats.seconds_run += since(t0);
         }

@@ -133,7 +133,6 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
         w.key = key;
     }
 
-    long host_bodies = 0;  // loop bodies launched by the host loop (use_graph = 0)
     HW_CUDA(cudaEventRecord(ctx->ev0, S.s));
     if (use_graph) {
         HW_CUDA(cudaGraphLaunch(w.init_exec, S.s));
@@ -142,7 +141,6 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
         S.enqueue_init(acc2, P.maxiters);
         for (int it = 0;; it++) {
             S.enqueue_body(0, 0);
-            host_bodies++;
             if ((it & 15) == 15) {
                 if ((rc = read_state(ctx)) != HW_OK) return rc;
                 if (ctx->cg_state_host->status != CG_RUNNING) break;
@@ -175,8 +173,7 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
         } else {
             for (int it = 0;; it++) {
                 S.enqueue_body(0, 0);
-                host_bodies++;
-                if ((it & 15) == 15) {
+                    if ((it & 15) == 15) {
                     if ((rc = read_state(ctx)) != HW_OK) return rc;
                     if (h->status != CG_RUNNING) break;
                 }
@@ -199,11 +196,11 @@ int run_f64(F64Solve &S, const hw_cg_params &P, hw_cg_result *R) {
         R->rr_relative = h->src_norm2 > 0 ? h->rr / h->src_norm2 : 0.0;
         R->true_residual = true_res;
         R->seconds = ms * 1e-3;
-        // kernels per phase: init = [2 for M^dag b] + 4 (A x0) + 1; body = 5; check = 2 (M x) or 4
+        // kernels per phase: init = [2 for M^dag b] + 4 (A x0) + 1; body = 5, in a host loop 6
+        // (k_pupdate_done); check = 2 (M x) or 4
         const long init_k = (S.mode == MODE_SOLVE ? 2 : 0) + 5;
         const long check_k = S.mode == MODE_SOLVE ? 2 : 4;
-        const long bodies = use_graph ? (long)h->iter + restarts + 1 : host_bodies;
-        R->kernel_launches = (int)(init_k + 5 * bodies + check_k * (1 + restarts));
+        R->kernel_launches = (int)(init_k + (use_graph ? 5L : 6L) * h->bodies + check_k * (1 + restarts));
         if (h->status == CG_BREAKDOWN)
             R->status = HW_ERR_BREAKDOWN;
         else if (h->status == CG_MAXITER || (P.true_residual && true_res > P.accuracy))

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kFullBlock, 4) k_full_hop(Geom g, Lk U, Full i
 }
 
 // p = r + beta p over both halves
-__global__ void __launch_bounds__(256) k_full_pupdate(long n, Full r, Full p, const CgState *st,
+__global__ void __launch_bounds__(256) k_full_pupdate(long n, Full r, Full p, CgState *st,
                                                      cudaGraphConditionalHandle cond) {
     if (blockIdx.x == 0 && threadIdx.x == 0) loop_next(st, cond, 1);
     if (!st->do_pupdate) return;
@@ -265,7 +265,7 @@ extern "C" int hw_wilson_cg_solve(const hw_gauge *gauge, double kappa, const hw_
         result->rr_relative = bb > 0 ? h->rr / bb : 0.0;
         result->true_residual = true_res;
         result->seconds = ms * 1e-3;
-        result->kernel_launches = 4 + 3 * std::max(h->iter, 1);
+        result->kernel_launches = 4 + 3 * h->bodies;
     }
     return status;
 }

@@ -17,7 +17,7 @@ namespace {
 
 int low_of(int precision) { return precision == HW_PREC_F16 ? LOW_F16 : LOW_F32; }
 
-void fill_result(const EngState &s, double seconds, int chunks, hw_cg_result *R) {
+void fill_result(const EngState &s, double seconds, unsigned long long launches, hw_cg_result *R) {
     std::memset(R, 0, sizeof(*R));
     R->iterations = s.iter;
     R->reliable_updates = s.n_ru;
@@ -25,9 +25,7 @@ void fill_result(const EngState &s, double seconds, int chunks, hw_cg_result *R)
     R->rr_relative = s.b2 > 0 ? s.rr / s.b2 : 0.0;
     R->true_residual = s.b2 > 0 ? std::sqrt(s.s2 / s.b2) : 0.0;
     R->seconds = seconds;
-    // every loop body launches P1..P4, the gate, P5 and the control kernel, a body with a
-    // reliable update its seven phases more; every chunk one kernel
-    R->kernel_launches = chunks + 7 * (s.iter + 1) + 7 * s.n_ru;
+    R->kernel_launches = (int)launches;
     if (s.status == ENG_CONVERGED)
         R->status = HW_OK;
     else if (s.status == ENG_BREAKDOWN)
@@ -76,7 +74,7 @@ int mixed_solve(const hw_gauge *G, double kappa, const hw_field *src, hw_field *
     float ms = 0;
     HW_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     hw_cg_result tmp;
-    fill_result(E->state(slot), ms * 1e-3, chunks, R ? R : &tmp);
+    fill_result(E->state(slot), ms * 1e-3, E->launches_of(slot), R ? R : &tmp);
     const int status = R ? R->status : tmp.status;
     E->release(slot);
     E->prune_lattices();
@@ -121,7 +119,7 @@ int drive_batch(hw_context *ctx, Engine *E, int n, long max_chunks, hw_cg_result
             if (done[k]) continue;
             const EngState &s = E->state(slot_of[k]);
             if (s.status == ENG_RUNNING) continue;
-            fill_result(s, now, chunks, &results[k]);
+            fill_result(s, now, E->launches_of(slot_of[k]), &results[k]);
             HW_CUDA(finished(k));
             E->release(slot_of[k]);
             done[k] = 1;

@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kStagBlock) k_stag_cg(Geom g, Lk U, int par, H
 }
 
 // p = r + beta p
-__global__ void __launch_bounds__(kStagVecBlock) k_stag_pupdate(int Vh, HalfStag r, HalfStag p, const CgState *st,
+__global__ void __launch_bounds__(kStagVecBlock) k_stag_pupdate(int Vh, HalfStag r, HalfStag p, CgState *st,
                                                                cudaGraphConditionalHandle cond) {
     if (blockIdx.x == 0 && threadIdx.x == 0) loop_next(st, cond, 1);
     if (!st->do_pupdate) return;
@@ -524,7 +524,7 @@ int hw_staggered_cg_solve(const hw_gauge *gauge, double mass, const hw_stag_fiel
         result->rr_relative = bb > 0 ? h->rr / bb : 0.0;
         result->true_residual = true_res;
         result->seconds = ms * 1e-3;
-        result->kernel_launches = 8 + 5 * std::max(h->iter, 1);
+        result->kernel_launches = 8 + 5 * h->bodies;
     }
     return status;
 }

@@ -219,7 +219,8 @@ typedef struct hw_cg_result {
                                it (conjugate_gradient.h:103) */
     double true_residual;   /* |b - A x| / |b| recomputed in FP64 */
     double seconds;         /* device time of the solve */
-    int kernel_launches;    /* CUDA kernels the solve launched (graph nodes included) */
+    int kernel_launches;    /* CUDA kernels that ran for the solve (graph nodes included); in a
+                             * batch those of the launches it shared with the others */
 } hw_cg_result;
 
 /* fill params with the reference defaults (accuracy 1e-12, maxiters 10000, FP64) */

@@ -160,3 +160,46 @@ def test_loop_graph_limits(hw, ctx, oracle, kind):
     assert r.converged and r.iterations == 0 and not x.any()
     r, _ = solve(good, zero, true_residual=True)
     assert r.converged and r.true_residual <= 1e-10
+
+
+def test_launch_counts(hw, ctx, oracle, monkeypatch):
+    """kernel_launches against the kernels that the loops are made of: start + bodies + check."""
+    dims = (4, 4, 4, 4)
+    U = oracle.gen_links(dims, 0.3, 5)
+
+    def system(c):
+        lat = hw.Lattice(c, dims)
+        G = hw.GaugeField(lat, U)
+        return lat, G, hw.Field(lat, oracle.gen_spinor(dims, 6, oracle.EVEN)), hw.Field(lat)
+
+    lat, G, b, x = system(ctx)
+    D, F, S = hw.Dirac_Wilson_evenodd(0.12, G), hw.Dirac_Wilson(0.12, G), hw.dirac_staggered_evenodd(4.0, G)
+    r = D.solve(b, x, accuracy=1e-10, maxiters=3)
+    assert r.iterations == 3 and r.kernel_launches == 7 + 5 * 3 + 2
+    x.zero()
+    r = D.solve(b, x, accuracy=1e-10, maxiters=3, use_graph=False)  # 16 bodies before the host looks
+    assert r.iterations == 3 and r.kernel_launches == 7 + 6 * 16 + 2
+    x.zero()
+    r = hw.CG(D, accuracy=1e-10).apply(b, x)
+    assert r.kernel_launches == 5 + 5 * r.iterations + 4
+    x.zero()
+    r = F.cg(b, x, accuracy=1e-10)
+    assert r.kernel_launches == 4 + 3 * r.iterations
+    sb, sx = hw.StaggeredField(lat, np.ones((lat.volume, 3, 2)), hw.EVEN), hw.StaggeredField(lat)
+    r = S.cg(sb, sx, accuracy=1e-10)
+    assert r.kernel_launches == 8 + 5 * r.iterations
+    # engine: per chunk 1, per body P1..P4, gate, P5, control, per update R1..R5L
+    for prec in ("f16", "f32"):
+        x.zero()
+        r = D.solve(b, x, accuracy=1e-10, precision=prec)
+        chunks = -(-(r.iterations + 1) // 64)
+        assert r.converged and r.kernel_launches == chunks + 7 * (r.iterations + 1) + 7 * r.reliable_updates
+    # a host loop launches every phase in all 64 iterations of a chunk, and no gate
+    monkeypatch.setenv("HW_USE_GRAPH", "0")
+    c = hw.Context(0)
+    lat, G, b, x = system(c)
+    r = hw.Dirac_Wilson_evenodd(0.12, G).solve(b, x, accuracy=1e-10, precision="f16")
+    chunks = -(-(r.iterations + 1) // 64)
+    assert r.converged and r.kernel_launches == chunks * (1 + 64 * 13)
+    lat.close()
+    c.close()

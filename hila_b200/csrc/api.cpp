@@ -179,7 +179,6 @@ int hw_context_destroy(hw_context *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     destroy_engines(ctx);
-    ctx->copier.reset();
     if (ctx->cg_state_host) cudaFreeHost(ctx->cg_state_host);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);

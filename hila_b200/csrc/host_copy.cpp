@@ -6,34 +6,30 @@
 // of its own, bring slices over and store them, so the bus, the stores and the page faults
 // overlap.  A force of 32 MB into a fresh array (1.8 ms of which are its page faults on one
 // thread): 5.9 -> 3.6 ms with its kernels; a staggered field of 16 MB: 2.06 -> 1.87 ms.
-#include <cuda_runtime.h>
+#include "host_copy.h"
 
 #include <algorithm>
 #include <cstring>
 #include <thread>
 
-#include "hw_internal.h"
-
 namespace hw {
-
-namespace {
-constexpr size_t kCopyChunk = 1 << 20;
-constexpr size_t kCopyMin = 2 << 20;  // smaller copies go the plain way
-}  // namespace
 
 HostCopier::~HostCopier() {
     for (int w = 0; w < kCopyWorkers; w++) {
-        if (stream[w]) cudaStreamDestroy(stream[w]);
-        if (buf[w]) cudaFreeHost(buf[w]);
+        if (stream_[w]) cudaStreamDestroy(stream_[w]);
+        if (buf_[w]) cudaFreeHost(buf_[w]);
     }
 }
 
-int HostCopier::init() {
-    for (int w = 0; w < kCopyWorkers; w++) {
-        if (!stream[w]) HW_CUDA(cudaStreamCreateWithFlags(&stream[w], cudaStreamNonBlocking));
-        if (!buf[w]) HW_CUDA(cudaMallocHost(&buf[w], kCopyChunk));
+int HostCopier::ready(int want) {
+    for (int w = 0; w < want; w++) {
+        if ((!stream_[w] && cudaStreamCreateWithFlags(&stream_[w], cudaStreamNonBlocking) != cudaSuccess) ||
+            (!buf_[w] && cudaMallocHost(&buf_[w], kCopyChunk) != cudaSuccess)) {
+            cudaGetLastError();  // the copy does without
+            return w;
+        }
     }
-    return HW_OK;
+    return want;
 }
 
 static bool pageable(const void *p) {
@@ -45,47 +41,44 @@ static bool pageable(const void *p) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-int copy_to_host(hw_context *ctx, void *dst, const void *src, size_t bytes) {
-    if (bytes >= kCopyMin && pageable(dst)) {
-        if (!ctx->copier) ctx->copier.reset(new HostCopier());
-        HostCopier &C = *ctx->copier;
-        int rc = C.init();
-        if (rc != HW_OK) return rc;
-        HW_CUDA(cudaStreamSynchronize(ctx->stream));  // the source is complete
-        const size_t chunks = (bytes + kCopyChunk - 1) / kCopyChunk;
-        const int n = (int)std::min<size_t>(kCopyWorkers, chunks);
-        cudaError_t err[kCopyWorkers] = {};
-        auto work = [&](int w) {
-            cudaError_t e = cudaSetDevice(ctx->device);
-            for (size_t c = w; c < chunks && e == cudaSuccess; c += n) {
-                const size_t off = c * kCopyChunk, len = std::min(kCopyChunk, bytes - off);
-                e = cudaMemcpyAsync(C.buf[w], (const char *)src + off, len, cudaMemcpyDeviceToHost, C.stream[w]);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(C.stream[w]);
-                if (e == cudaSuccess) std::memcpy((char *)dst + off, C.buf[w], len);
-            }
-            err[w] = e;
-        };
-        std::thread th[kCopyWorkers];
-        bool started[kCopyWorkers] = {};
-        for (int w = 1; w < n; w++) {
-            try {
-                th[w] = std::thread(work, w);
-                started[w] = true;
-            } catch (...) {  // no thread to be had: its slices are copied here below
-            }
-        }
-        work(0);
-        for (int w = 1; w < n; w++) {
-            if (started[w])
-                th[w].join();
-            else
-                work(w);
-        }
-        for (int w = 0; w < n; w++) HW_CUDA(err[w]);
+int HostCopier::copy(int device, cudaStream_t s, void *dst, const void *src, size_t bytes) {
+    const size_t chunks = (bytes + kCopyChunk - 1) / kCopyChunk;
+    int n = 0;
+    if (bytes >= kCopyMin && pageable(dst)) n = ready((int)std::min<size_t>(kCopyWorkers, chunks));
+    if (n < 2) {
+        HW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+        HW_CUDA(cudaStreamSynchronize(s));
         return HW_OK;
     }
-    HW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    HW_CUDA(cudaStreamSynchronize(ctx->stream));
+    HW_CUDA(cudaStreamSynchronize(s));  // the source is complete
+    cudaError_t err[kCopyWorkers] = {};
+    auto work = [&](int w) {
+        cudaError_t e = cudaSetDevice(device);
+        for (size_t c = w; c < chunks && e == cudaSuccess; c += n) {
+            const size_t off = c * kCopyChunk, len = std::min(kCopyChunk, bytes - off);
+            e = cudaMemcpyAsync(buf_[w], (const char *)src + off, len, cudaMemcpyDeviceToHost, stream_[w]);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream_[w]);
+            if (e == cudaSuccess) std::memcpy((char *)dst + off, buf_[w], len);
+        }
+        err[w] = e;
+    };
+    std::thread th[kCopyWorkers];
+    bool started[kCopyWorkers] = {};
+    for (int w = 1; w < n; w++) {
+        try {
+            th[w] = std::thread(work, w);
+            started[w] = true;
+        } catch (...) {  // no thread to be had: its slices are copied here below
+        }
+    }
+    work(0);
+    for (int w = 1; w < n; w++) {
+        if (started[w])
+            th[w].join();
+        else
+            work(w);
+    }
+    for (int w = 0; w < n; w++) HW_CUDA(err[w]);
     return HW_OK;
 }
 

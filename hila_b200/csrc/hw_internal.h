@@ -12,6 +12,7 @@
 
 #include "errors.h"
 #include "graph_build.h"
+#include "host_copy.h"
 #include "kernels.h"
 
 namespace hw {
@@ -34,16 +35,6 @@ struct DevBuf {
     }
 };
 
-// Threads, page-locked chunks and streams of the copies into pageable memory (host_copy.cpp),
-// kept by the context (8 MiB)
-constexpr int kCopyWorkers = 8;
-struct HostCopier {
-    void *buf[kCopyWorkers] = {};
-    cudaStream_t stream[kCopyWorkers] = {};
-    int init();
-    ~HostCopier();
-};
-
 // Sites per parity rounded up to 64 so every SoA plane starts 1 KiB aligned
 // (for FP64 planes) and coalesced rows never straddle planes.
 inline int padded_stride(long vh) { return (int)((vh + 63) / 64 * 64); }
@@ -62,7 +53,7 @@ struct hw_context {
     hw::DevBuf stage;         // lexicographic staging buffer for host transfers (grow-only)
     hw::CgState *cg_state_host = nullptr;  // pinned mirror
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    std::unique_ptr<hw::HostCopier> copier;  // made by the first large copy into pageable memory
+    hw::HostCopier copier;  // copies into pageable memory
     hw::RedBuf red() const {
         return hw::RedBuf{red_partials.as<double>(), red_ticket.as<unsigned>(), red_capacity_doubles};
     }
@@ -172,6 +163,8 @@ inline int force_buffer(hw_context *ctx, size_t bytes, DevBuf &own, void **out) 
 }
 // device -> host after the work on the context's stream; returns when dst is complete.  The
 // caller holds the context's lock.
-int copy_to_host(hw_context *ctx, void *dst, const void *src, size_t bytes);
+inline int copy_to_host(hw_context *ctx, void *dst, const void *src, size_t bytes) {
+    return ctx->copier.copy(ctx->device, ctx->stream, dst, src, bytes);
+}
 void destroy_engines(hw_context *ctx);
 }  // namespace hw

@@ -2,7 +2,7 @@
 reductions (hila_b200/csrc/hop_shapes.h) by tests/cpp/test_reductions.cpp, the division of the
 engine's tiles (engine_parts.h) by test_parts.cpp, graph construction (graph_build.h) over a
 fake CUDA runtime by test_graph_build.cpp, the cache of graphs (graph_cache.h) by
-test_graph_cache.cpp."""
+test_graph_cache.cpp, copies into pageable memory over a fake runtime by test_host_copy.cpp."""
 import os
 import subprocess
 
@@ -37,3 +37,8 @@ def test_graph_build(tmp_path):
 
 def test_graph_cache(tmp_path):
     assert "graph cache passed" in compile_and_run(tmp_path, "test_graph_cache")
+
+
+def test_host_copy(tmp_path):
+    assert "host copies passed" in compile_and_run(tmp_path, "test_host_copy", os.path.join(CSRC, "host_copy.cpp"),
+                                                   "-I", CUDA_INCLUDE, "-pthread")

@@ -493,6 +493,20 @@ CgWorkspace::~CgWorkspace() {
 
 LoopCgWorkspace::~LoopCgWorkspace() {
     if (loop_exec) cudaGraphExecDestroy(loop_exec);
+    *total -= kept;
+}
+
+LoopCgLease::~LoopCgLease() {
+    if (!ws || (done && ws->kept)) return;
+    size_t bytes = ws->t.bytes;
+    for (int h = 0; h < 2; h++)
+        for (const hw::DevBuf *d : {&ws->r[h], &ws->p[h], &ws->Dp[h], &ws->x[h]}) bytes += d->bytes;
+    if (done && (*ws->total += bytes) <= kLoopWsKeep) {
+        ws->kept = bytes;
+        return;
+    }
+    if (done) *ws->total -= bytes;
+    ws.reset();
 }
 
 hw_lattice::~hw_lattice() {

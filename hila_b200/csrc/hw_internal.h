@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <memory>
@@ -54,6 +55,7 @@ struct hw_context {
     hw::CgState *cg_state_host = nullptr;  // pinned mirror
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     hw::HostCopier copier;  // copies into pageable memory
+    std::shared_ptr<std::atomic<size_t>> loop_ws_bytes = std::make_shared<std::atomic<size_t>>(0);
     hw::RedBuf red() const {
         return hw::RedBuf{red_partials.as<double>(), red_ticket.as<unsigned>(), red_capacity_doubles};
     }
@@ -93,8 +95,13 @@ struct CgWorkspace {
 
 // Workspace of a CG over device fields that keeps its loop graph (solver_full.cu,
 // staggered.cu): the iterated fields and the solution are the workspace's own, so the graph
-// serves every source and solution on the lattice.
+// serves every source and solution on the lattice.  After a call it stays with its lattice while
+// the context's lattices keep no more than kLoopWsKeep bytes together (a Wilson 32^4 has 0.8 GB),
+// else it is freed.
+constexpr size_t kLoopWsKeep = size_t(1) << 30;
 struct LoopCgWorkspace {
+    std::shared_ptr<std::atomic<size_t>> total;  // bytes kept by the context's workspaces
+    size_t kept = 0;                             // of them, this one's
     hw::DevBuf r[2], p[2], Dp[2], x[2], t;  // [0] EVEN, [1] ODD (unpreconditioned solve only)
     cudaGraphExec_t loop_exec = nullptr;
     struct Key {
@@ -105,7 +112,16 @@ struct LoopCgWorkspace {
             return links == o.links && red == o.red && planes == o.planes && par == o.par;
         }
     } key;
+    explicit LoopCgWorkspace(std::shared_ptr<std::atomic<size_t>> t) : total(std::move(t)) {}
     ~LoopCgWorkspace();
+};
+
+// Frees a workspace at the end of the call that used it unless it may stay; after an error it is
+// freed in any case, as it may be half made.
+struct LoopCgLease {
+    std::unique_ptr<LoopCgWorkspace> &ws;
+    bool done = false;  // set when the call has come to its end
+    ~LoopCgLease();
 };
 
 struct hw_field;

@@ -203,7 +203,8 @@ extern "C" int hw_wilson_cg_solve(const hw_gauge *gauge, double kappa, const hw_
     HW_CUDA(cudaSetDevice(ctx->device));
     int rc;
     if ((rc = ensure_reduction_capacity(ctx, 2 * ((lat->Vh + kFullBlock - 1) / kFullBlock))) != HW_OK) return rc;
-    if (!lat->full_ws) lat->full_ws.reset(new LoopCgWorkspace());
+    if (!lat->full_ws) lat->full_ws.reset(new LoopCgWorkspace(ctx->loop_ws_bytes));
+    LoopCgLease lease{lat->full_ws};
     LoopCgWorkspace &w = *lat->full_ws;
     const size_t hb = (size_t)12 * lat->stride * sizeof(double2);
     cudaStream_t s = ctx->stream;
@@ -249,6 +250,7 @@ extern "C" int hw_wilson_cg_solve(const hw_gauge *gauge, double kappa, const hw_
     CgState *h = ctx->cg_state_host;
     HW_CUDA(cudaMemcpyAsync(h, st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
     HW_CUDA(cudaStreamSynchronize(s));
+    lease.done = true;
     const double bb = h->src_norm2;
     const double true_res = bb > 0 ? std::sqrt(h->res_num2 / bb) : 0.0;
     int status = h->status == CG_BREAKDOWN ? HW_ERR_BREAKDOWN

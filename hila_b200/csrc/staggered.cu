@@ -294,9 +294,9 @@ int check_stag_op(const hw_gauge *G, const hw_stag_field *a, const hw_stag_field
     return HW_OK;
 }
 
-// the lattice's staggered workspace (five half-lattice fields), kept with the lattice
+// the lattice's staggered workspace (five half-lattice fields); the caller holds a lease on it
 int ensure_stag_ws(hw_lattice *lat) {
-    if (!lat->stag_ws) lat->stag_ws.reset(new LoopCgWorkspace());
+    if (!lat->stag_ws) lat->stag_ws.reset(new LoopCgWorkspace(lat->ctx->loop_ws_bytes));
     LoopCgWorkspace &w = *lat->stag_ws;
     int rc;
     for (DevBuf *d : {&w.r[0], &w.p[0], &w.Dp[0], &w.x[0], &w.t})
@@ -419,6 +419,7 @@ int hw_staggered_evenodd_force(const hw_gauge *gauge, double mass, const hw_stag
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     HW_CUDA(cudaSetDevice(ctx->device));
     const int stride = lat->stride;
+    LoopCgLease lease{lat->stag_ws};
     if ((rc = ensure_stag_ws(lat)) != HW_OK) return rc;
     DevBuf own;
     void *out = nullptr;
@@ -436,7 +437,9 @@ int hw_staggered_evenodd_force(const hw_gauge *gauge, double mass, const hw_stag
         k_stag_force<-1><<<grid, kStagBlock, 0, ctx->stream>>>(lat->g, half_of(chi, 0), half_of(psi, 0), h1, h2,
                                                                lat->V, static_cast<double2 *>(out));
     HW_CUDA(cudaGetLastError());
-    return copy_to_host(ctx, force, out, bytes);
+    rc = copy_to_host(ctx, force, out, bytes);
+    lease.done = rc == HW_OK;
+    return rc;
 }
 
 // CG<dirac_staggered_evenodd>::apply (conjugate_gradient.h:46-104): M^dag M out = in
@@ -457,6 +460,7 @@ int hw_staggered_cg_solve(const hw_gauge *gauge, double mass, const hw_stag_fiel
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     HW_CUDA(cudaSetDevice(ctx->device));
     if ((rc = ensure_reduction_capacity(ctx, (lat->Vh + kStagBlock - 1) / kStagBlock)) != HW_OK) return rc;
+    LoopCgLease lease{lat->stag_ws};
     if ((rc = ensure_stag_ws(lat)) != HW_OK) return rc;
     LoopCgWorkspace &w = *lat->stag_ws;
     const int stride = lat->stride;
@@ -508,6 +512,7 @@ int hw_staggered_cg_solve(const hw_gauge *gauge, double mass, const hw_stag_fiel
     CgState *h = ctx->cg_state_host;
     HW_CUDA(cudaMemcpyAsync(h, st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
     HW_CUDA(cudaStreamSynchronize(s));
+    lease.done = true;
     const double bb = h->src_norm2;
     const double true_res = bb > 0 ? std::sqrt(h->res_num2 / bb) : 0.0;
     int status = h->status == CG_BREAKDOWN ? HW_ERR_BREAKDOWN

@@ -203,3 +203,32 @@ def test_launch_counts(hw, ctx, oracle, monkeypatch):
     assert r.converged and r.kernel_launches == chunks * (1 + 64 * 13)
     lat.close()
     c.close()
+
+
+def test_workspaces_are_given_back(hw, ctx):
+    """The workspaces that the loop-graph solvers keep with their lattices stay within 1 GiB
+    together (ten lattices of 123 MB each here), and go with the lattices."""
+    import torch
+    dims = (20, 20, 20, 20)
+    U = np.zeros((4, 20 ** 4, 3, 3, 2))
+    U[:, :, range(3), range(3), 0] = 1.0
+    b = np.ones((20 ** 4, 4, 3, 2))
+    c = hw.Context(0)
+    lats, before = [], None
+    for k in range(11):
+        lat = hw.Lattice(c, dims)
+        G, fb, fx = hw.GaugeField(lat, U), hw.Field(lat, b), hw.Field(lat)
+        lats.append((lat, hw.Dirac_Wilson(0.1, G), fb, fx))
+        if k == 0:  # what a first solve makes besides its workspace
+            lats[0][1].cg(fb, fx, maxiters=1)
+            lats[0][0].close()
+    before = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        for lat, D, fb, fx in lats[1:]:
+            assert D.cg(fb, fx, maxiters=1).status in (hw.HW_OK, hw.HW_ERR_NOT_CONVERGED)
+    kept = before - torch.cuda.mem_get_info()[0]
+    assert 0.5 * 2 ** 30 <= kept <= 2 ** 30 + 64 * 2 ** 20
+    for lat, *_ in lats[1:]:
+        lat.close()
+    assert torch.cuda.mem_get_info()[0] >= before
+    c.close()

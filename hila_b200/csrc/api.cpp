@@ -29,6 +29,7 @@ int DevBuf::alloc(size_t n) {
     cudaError_t e = cudaMalloc(&ptr, n);
     if (e != cudaSuccess) {
         ptr = nullptr;
+        cudaGetLastError();  // reported here, not by the next launch's check too
         set_error("cudaMalloc(%zu bytes) failed: %s", n, cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? HW_ERR_OOM : HW_ERR_CUDA;
     }

@@ -232,3 +232,17 @@ def test_workspaces_are_given_back(hw, ctx):
         lat.close()
     assert torch.cuda.mem_get_info()[0] >= before
     c.close()
+
+
+def test_out_of_memory_is_reported_once(hw, ctx, oracle):
+    """A field that no device holds (204 GB a half) fails by itself; calls after it do not."""
+    lat = hw.Lattice(ctx, (4, 4, 4, 4))
+    D = hw.Dirac_Wilson_evenodd(0.12, hw.GaugeField(lat, oracle.gen_links((4, 4, 4, 4), 0.3, 5)))
+    a, b = hw.Field(lat, oracle.gen_spinor((4, 4, 4, 4), 6, oracle.EVEN)), hw.Field(lat)
+    D.apply(a, b)
+    huge = hw.Lattice(ctx, (208, 200, 200, 256))
+    with pytest.raises(hw.HilaError) as e:
+        hw.Field(huge)
+    assert e.value.code == hw.HW_ERR_OOM
+    D.apply(a, b)
+    huge.close()

@@ -83,7 +83,7 @@ def test_cg_limits(hw, ctx, oracle):
     assert runs[0] == runs[1]
 
 
-@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 2, 4, 10), (8, 8, 8, 8)])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 2, 4, 10), (8, 8, 8, 8), (18, 14, 10, 22), (24, 24, 24, 20)])
 @pytest.mark.parametrize("link_format", [18, 12])
 def test_loop_graph_solvers(hw, ctx, oracle, dims, link_format):
     """Several sources, solutions, couplings and gauge fields on one lattice share a workspace and

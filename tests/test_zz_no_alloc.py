@@ -93,6 +93,45 @@ def test_noalloc_matches_evenodd_apply(hw, ctx, oracle, link_format, antiperiodi
         h.close()
 
 
+def test_noalloc_under_capture(hw, ctx, oracle):
+    """Calls captured into a CUDA graph, between the caller's own kernels (their launches overlap, so
+    the graph holds programmatic edges): replays give what the calls give, also on new inputs."""
+    import torch
+    dims, kappa = (6, 4, 8, 10), 0.124
+    V = int(np.prod(dims))
+    stride, idx = V // 2, eo_index(dims)
+    dev = torch.device("cuda:0")
+    links = torch.from_numpy(np.ascontiguousarray(link_planes(oracle.gen_links(dims, 0.3, 77), idx, stride))).to(dev)
+    a, b, c = (torch.zeros((12, stride, 2), dtype=torch.float64, device=dev) for _ in range(3))
+
+    def put(seed):
+        a.copy_(torch.from_numpy(spinor_planes(oracle.gen_spinor(dims, seed, oracle.EVEN), idx[0], stride)))
+
+    def chain():
+        a.mul_(2.0)
+        for src, dst, sign in ((a, b, 1), (b, c, -1)):
+            hw.wilson_evenodd_apply_noalloc(dims, kappa, sign, links.data_ptr(), src.data_ptr(), dst.data_ptr(), stride,
+                                            stream=torch.cuda.current_stream().cuda_stream)
+        c.add_(a)
+
+    put(1)
+    chain()  # outside a graph first: kernels are loaded
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for seed in (78, 79, 80):
+        put(seed)
+        chain()
+        torch.cuda.synchronize()
+        want = c.clone()
+        put(seed)
+        c.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(c, want) and bool(want.abs().sum() > 0)
+
+
 def test_noalloc_rejects_large_lattice(hw, ctx):
     with pytest.raises(hw.HilaError) as e:
         hw.wilson_evenodd_apply_noalloc((16, 16, 16, 18), 0.12, 1, 0x1000, 0x1000, 0x1000, 1 << 20)

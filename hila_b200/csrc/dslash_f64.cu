@@ -324,7 +324,7 @@ __device__ __forceinline__ void sum_terms(const SplitTerms &part, int lane, Cx<d
 // forward or backward) of the block's sites, the half spinors meet in shared memory, and warp
 // s < 4 sums spin s, in the order of hop_site, and runs the epilogue on it.  A site's loads
 // are all in flight together, where k_hop's thread goes through eight dependent rounds of
-// them, and a lattice of some thousand sites reaches eight times as many SMs.
+// them, and a lattice of some thousand sites makes four times as many blocks.
 template <int SIGN, class Lk, class Epi>
 __global__ void __launch_bounds__(kSplitBlock, 2) k_hop_split(Geom g, Lk U, int par, SpinorF64 in, Epi epi,
                                                              RedBuf red) {

@@ -123,7 +123,10 @@ struct FullResidual {
     __device__ void operator()(const double *tot) { st->res_num2 = tot[0]; }
 };
 
-// the hop over both parities: blocks [0, n) EVEN output sites, [n, 2n) ODD ones
+// the hop over both parities: blocks [0, n) EVEN output sites, [n, 2n) ODD ones.  At most 128
+// registers, for four blocks per SM: us per iteration (18-real links) without the bound -> with
+// it, 12^4 36 -> 36, 16^4 91 -> 64 (one wave of blocks), 20^4 203 -> 207, 24^4 405 -> 374, 32^4
+// 1233 -> 1087; 12 reals alike (32^4 991 -> 888).
 template <int SIGN, class Lk, class Epi>
 __global__ void __launch_bounds__(kFullBlock, 4) k_full_hop(Geom g, Lk U, Full in, Epi epi, RedBuf red) {
     if (epi.skip()) return;

@@ -313,11 +313,17 @@ class PinnedArray:
 
 # ------------------------------------------------------------------ handles
 
+def _release(handle, destroy) -> None:
+    """Destroy what a handle points to and clear it in place, for everyone who holds it."""
+    if handle:
+        destroy(handle)
+        handle.value = None
+
+
 def _close_children(children):
-    for ref in reversed(children):
-        obj = ref()
-        if obj is not None:
-            obj.close()
+    for handle, destroy in reversed(children):
+        _release(handle, destroy)
+    children.clear()
 
 
 class Context:
@@ -325,7 +331,8 @@ class Context:
 
     Handles made on a context (lattices, gauge and spinor fields, servers)
     register here; close() releases them first, newest first, so no handle can
-    reach the C context after it is gone."""
+    reach the C context after it is gone.  The parents hold the handles themselves:
+    the garbage collector may end a cycle's parent before its children."""
 
     def __init__(self, device: int = 0):
         self.handle = _vp()
@@ -333,9 +340,8 @@ class Context:
         self.device = device
         self._children = []
 
-    def _adopt(self, obj):
-        import weakref
-        self._children.append(weakref.ref(obj))
+    def _adopt(self, handle, destroy):
+        self._children.append((handle, destroy))
 
     def synchronize(self):
         _check(lib().hw_context_synchronize(self.handle))
@@ -381,9 +387,7 @@ class Context:
     def close(self):
         if self.handle:
             _close_children(self._children)
-            self._children = []
-            lib().hw_context_destroy(self.handle)
-            self.handle = _vp()
+            _release(self.handle, lib().hw_context_destroy)
 
     def __del__(self):
         try:
@@ -404,19 +408,16 @@ class Lattice:
         _check(lib().hw_lattice_create(ctx.handle, _dims(self.dims), int(bool(antiperiodic)),
                                        ctypes.byref(self.handle)))
         self._children = []
-        ctx._adopt(self)
+        ctx._adopt(self.handle, lib().hw_lattice_destroy)
 
-    def _adopt(self, obj):
-        import weakref
-        self._children.append(weakref.ref(obj))
-        self.ctx._adopt(obj)
+    def _adopt(self, handle, destroy):
+        self._children.append((handle, destroy))
+        self.ctx._adopt(handle, destroy)
 
     def close(self):
         if self.handle:
             _close_children(self._children)
-            self._children = []
-            lib().hw_lattice_destroy(self.handle)
-            self.handle = _vp()
+            _release(self.handle, lib().hw_lattice_destroy)
 
     def __del__(self):
         try:
@@ -436,12 +437,10 @@ class GaugeField:
         self.link_format = link_format
         self.handle = _vp()
         _check(lib().hw_gauge_create(lattice.handle, _dptr(links), int(link_format), ctypes.byref(self.handle)))
-        lattice._adopt(self)
+        lattice._adopt(self.handle, lib().hw_gauge_destroy)
 
     def close(self):
-        if self.handle:
-            lib().hw_gauge_destroy(self.handle)
-            self.handle = _vp()
+        _release(self.handle, lib().hw_gauge_destroy)
 
     def __del__(self):
         try:
@@ -457,7 +456,7 @@ class Field:
         self.lattice = lattice
         self.handle = _vp()
         _check(lib().hw_field_create(lattice.handle, ctypes.byref(self.handle)))
-        lattice._adopt(self)
+        lattice._adopt(self.handle, lib().hw_field_destroy)
         if data is not None:
             self.upload(data, parity)
 
@@ -496,9 +495,7 @@ class Field:
         _check(lib().hw_field_zero(self.handle, int(parity)))
 
     def close(self):
-        if self.handle:
-            lib().hw_field_destroy(self.handle)
-            self.handle = _vp()
+        _release(self.handle, lib().hw_field_destroy)
 
     def __del__(self):
         try:
@@ -566,7 +563,7 @@ class StaggeredField:
         self.lattice = lattice
         self.handle = _vp()
         _check(lib().hw_stag_field_create(lattice.handle, ctypes.byref(self.handle)))
-        lattice._adopt(self)
+        lattice._adopt(self.handle, lib().hw_stag_field_destroy)
         if data is not None:
             self.upload(data, parity)
 
@@ -585,9 +582,7 @@ class StaggeredField:
         _check(lib().hw_stag_field_zero(self.handle, int(parity)))
 
     def close(self):
-        if self.handle:
-            lib().hw_stag_field_destroy(self.handle)
-            self.handle = _vp()
+        _release(self.handle, lib().hw_stag_field_destroy)
 
     def __del__(self):
         try:
@@ -880,7 +875,7 @@ class Server:
         self.ctx = ctx
         self.handle = _vp()
         _check(lib().hw_server_create(ctx.handle, ctypes.byref(cfg), ctypes.byref(self.handle)))
-        ctx._adopt(self)
+        ctx._adopt(self.handle, lib().hw_server_destroy)
 
     def add_gauge(self, gauge: GaugeField) -> int:
         gid = ctypes.c_int()
@@ -963,9 +958,7 @@ class Server:
         return {f: getattr(st, f) for f, _ in _ServerStats._fields_}
 
     def close(self):
-        if self.handle:
-            lib().hw_server_destroy(self.handle)
-            self.handle = _vp()
+        _release(self.handle, lib().hw_server_destroy)
 
     def __del__(self):
         try:

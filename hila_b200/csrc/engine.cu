@@ -561,7 +561,8 @@ __global__ void __launch_bounds__(kEngTile, MINB) k_eng_low(EngPtrs P) {
             }
         }
         __syncthreads();  // s_act is rewritten by the next item
-        if constexpr (NRED > 0) arrive_and_finish<PHASE, NRED>(P, La, l, smem, last, PARTS ? TP.items(La.ntiles) : La.ntiles);
+        if constexpr (NRED > 0)
+            arrive_and_finish<PHASE, NRED>(P, La, l, smem, last, PARTS ? TP.items(La.ntiles) : La.ntiles);
     }
 }
 
@@ -729,7 +730,8 @@ __global__ void __launch_bounds__(kEngTile) k_eng_vec(EngPtrs P) {
 // running slots, and keeps the chunk's WHILE loop going while some slot runs
 // and fewer than `chunk` iterations ran.  No waiting: the loop is bounded by
 // `chunk` and by every slot's maxiter.
-__global__ void k_eng_control(EngPtrs P, int nprob, int chunk, int kernels, int ru_kernels, cudaGraphConditionalHandle h, int use_cond) {
+__global__ void k_eng_control(EngPtrs P, int nprob, int chunk, int kernels, int ru_kernels,
+                              cudaGraphConditionalHandle h, int use_cond) {
     __shared__ int running;
     if (threadIdx.x == 0) running = 0;
     __syncthreads();

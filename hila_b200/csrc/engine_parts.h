@@ -24,7 +24,7 @@ namespace hw {
 constexpr int kPartsUnitCost = 4;
 constexpr int kPartsOverheadF32 = 1, kPartsOverheadF16 = 3, kPartsOverheadPair = 4;
 constexpr int kPartsEmptyCost = 1;  // an item without slots
-constexpr int kPartsGroups = 16;
+constexpr int kPartsGroups = 16;    // in which a lattice's uneven parts alternate (parts_time)
 
 struct PartsLattice {
     int ntiles;
@@ -60,8 +60,9 @@ inline bool parts_even(const PartsLattice *lat, int nlat, const PartsShape &S, i
 // When the launch ends: the mean of two reckonings, as the truth lies between them.  One takes the
 // items in turn by the next free block, each at its full cost (whole waves); the other lets the
 // last, partly filled wave run faster (the work spread over all blocks and half an item).  A launch
-// of one wave ends with its longest item.  Times are below kPartsTimes for up to two tiles per block of up to 16 slots (a tile
-// costs up to 16 x (kPartsUnitCost + overhead)).  Some microseconds on the host.
+// of one wave ends with its longest item.  Times are below kPartsTimes for up to two tiles per
+// block of up to 16 slots (a tile costs up to 16 x (kPartsUnitCost + overhead)).  Takes some
+// microseconds on the host.
 constexpr int kPartsTimes = 512;
 inline double parts_time(const PartsLattice *lat, int nlat, const PartsShape &S, int parts) {
     long free_at[kPartsTimes] = {S.blocks};  // blocks that become free then
